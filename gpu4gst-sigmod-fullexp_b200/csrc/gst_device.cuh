@@ -165,7 +165,7 @@ struct Ctx {
                        // frontier as they stood when the round began (V rows of ds)
   uint32_t* dist_h;    // hop budgets h = 1..nhb: d_i^{<=h}(v), cheapest paths of at most h
                        // edges (nhb x V rows of ds; budget D is dist itself)
-  uint32_t* tour;      // 2^k x TOUR_STRIDE path table, then 2^k x KMAX row minima
+  uint32_t* tour;      // 2^k x TOUR_STRIDE path table, 2^k x KMAX row minima, 2^k rest bounds
   uint4* q[2];
   uint4* far[2];
   uint32_t* rows;
@@ -372,15 +372,18 @@ __device__ __forceinline__ uint32_t sssp_cutoff(const Ctx* c) {
   return x >= COST_INF ? COST_INF : (uint32_t)x;
 }
 
-// Largest edge weight a grow step from a state of cost `cost` can still use: a
-// target must stay <= ub (unbounded) or < ub_cell (hop-bounded).
-__device__ __forceinline__ uint32_t grow_limit(const Ctx* c, uint32_t cost) {
-  if (c->hop) {
-    const uint32_t b = c->ub_cell;
-    return b > cost ? b - cost - 1u : 0u;
-  }
-  const uint32_t b = c->ub;
-  return b >= cost ? b - cost : 0u;
+// Rest bounds of a query (build_tour): entry X is a lower bound of any tree that covers
+// the groups of X, wherever it hangs.
+__device__ __forceinline__ const uint32_t* rest_bounds(const Ctx* c) {
+  return c->tour + (size_t)c->W * (TOUR_STRIDE + KMAX);
+}
+// Largest edge weight a grow step from a state of cost `cost` can still use when the
+// groups it misses cost at least `rest` more: the tree must stay <= bound (unbounded) or
+// < bound (hop-bounded).
+__device__ __forceinline__ uint32_t grow_limit(bool hop, uint32_t bound, uint32_t cost,
+                                               uint32_t rest) {
+  const uint64_t used = (uint64_t)cost + rest + (hop ? 1u : 0u);
+  return (uint64_t)bound > used ? (uint32_t)(bound - used) : 0u;
 }
 
 __device__ __forceinline__ void mark_row(Ctx* c, uint32_t u) {
@@ -972,7 +975,7 @@ __global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G
   const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   for (uint32_t base = wid * 32; base < total; base += warps * 32) {
     const uint32_t it = base + lane;
-    uint32_t v = 0, pd = 0, cost = 0, bound = 0, e_off = 0;
+    uint32_t v = 0, pd = 0, cost = 0, bound = 0, e_off = 0, wmax = 0;
     bool chunk = false;
     int qi = 0;
     Plan P{0, 0u, false, false, 0u, 0u, 0u};
@@ -995,8 +998,13 @@ __global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G
       // a work item always names a state that holds a finite cost
       const bool src_ok = !ok || in_bounds(c, cost_of(cell) != COST_INF, 12);
       if (ok && src_ok && cost_of(cell) >= cost && 2ull * cost <= (uint64_t)bound) {
-        const uint32_t wmax = c->hop ? (bound > cost ? bound - cost - 1u : 0u)
-                                     : (bound >= cost ? bound - cost : 0u);
+        // The missing groups cost at least the rest bound wherever the tree goes on, so
+        // heavier edges than this one lead to no tree within the bound.  The kernel is
+        // bound by the random row each relaxation reads (300 relaxations per state
+        // written); on 32 queries of k = 5/7 over 141k vertices the limit cuts 973 M of
+        // them to 61 M, 20.8 to 6.2 ms, on the 4M-vertex batch 2172 M to 327 M, 45.7 to
+        // 18.6 ms.
+        wmax = grow_limit(c->hop, bound, cost, c->use_tour ? __ldg(&rest_bounds(c)[(uint32_t)c->full ^ p]) : 0u);
         P = plan_item(G, v, b0, b1, cost, e.w, wmax, c->bucket_end, split, chunk);
       }
     }
@@ -1010,7 +1018,7 @@ __global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G
     const uint32_t tot = __shfl_sync(0xffffffffu, scan, 31);
     for (uint32_t j0 = 0; j0 < tot; j0 += 32 * RELAX_U) {
       int2 ed[RELAX_U];
-      uint32_t x_v[RELAX_U], x_pd[RELAX_U], x_cost[RELAX_U], x_bound[RELAX_U];
+      uint32_t x_v[RELAX_U], x_pd[RELAX_U], x_cost[RELAX_U], x_bound[RELAX_U], x_wmax[RELAX_U];
       uint64_t cur[RELAX_U];
       int x_qi[RELAX_U];
       bool ok[RELAX_U];
@@ -1025,6 +1033,7 @@ __global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G
         x_pd[x] = __shfl_sync(0xffffffffu, pd, o);
         x_cost[x] = __shfl_sync(0xffffffffu, cost, o);
         x_bound[x] = __shfl_sync(0xffffffffu, bound, o);
+        x_wmax[x] = __shfl_sync(0xffffffffu, wmax, o);
         x_qi[x] = __shfl_sync(0xffffffffu, qi, o);
         const uint32_t off = j - (o_scan - o_n);
         ok[x] = j < tot && in_bounds(ctxs + x_qi[x], o_eb + off < G.E, 6);
@@ -1042,10 +1051,10 @@ __global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G
 #pragma unroll
       for (int x = 0; x < RELAX_U; x++) {
         Ctx* c = ctxs + x_qi[x];
-        const uint32_t u = (uint32_t)ed[x].x, nc = x_cost[x] + (uint32_t)ed[x].y;
-        // a target costing more than ub cannot be part of an optimal tree
+        const uint32_t u = (uint32_t)ed[x].x;
+        // heavier than the item's limit: no tree within the bound
         const int hop = c->hop;
-        const bool keep = hop ? (nc < x_bound[x]) : (nc <= x_bound[x]);
+        const bool keep = (uint32_t)ed[x].y <= x_wmax[x];
         const uint32_t d = (x_pd[x] >> 16) + (uint32_t)hop;
         ok[x] = ok[x] && in_bounds(c, u < G.V, 7) && keep && in_bounds(c, d < (uint32_t)c->DD, 11);
         rm[x] = ok[x] && c->rowmap ? __ldcg(&c->rowmap[u]) : ROW_NONE;
@@ -1205,6 +1214,7 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
     if (lane == 0) atomicAnd(&c->rowbits[v >> 5], ~(1u << (v & 31)));
     __syncwarp();
     const uint32_t ubm = hop ? c->ub_cell : c->ub;
+    const uint32_t* rest = c->use_tour ? rest_bounds(c) : nullptr;
     // Merge closure T(v, X|Y) <= T(v, X) + T(v, Y), by rounds of popcount class: in a
     // round the unprocessed pending cells X of the smallest class (clist) are merged
     // with every finite cell Y disjoint from them, all pairs of the round spread
@@ -1269,7 +1279,11 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
           const uint32_t cand = cost_of(B(cell)) + cy;
           bool ok = cy != COST_INF && !(hop && (int)(d1 + d2) > D) &&
                     in_bounds(c, yi < (uint32_t)RW && S < (uint32_t)W, 9);
-          if (ok && S != full && 3ull * cand > 2ull * ubm) ok = false;
+          // (the rest bound drops 3 of 4 pairs' results on the batches above: 1426 M
+          // pairs become 240 M, 47 to 28 ms at 4M vertices)
+          if (ok && S != full &&
+              (3ull * cand > 2ull * ubm || (uint64_t)cand + (rest ? __ldg(&rest[full ^ S]) : 0u) + hop > ubm))
+            ok = false;
           if (ok) {
             const uint32_t nd = d1 > d2 ? d1 : d2;
             tgt = (nd << k) + S;
@@ -1534,6 +1548,10 @@ __device__ __forceinline__ void ctrl_take_far(Ctx* c) {
 // row minima P2[X][i] = min_j P[X][i][j].  The reference builds a closure of the
 // same table on the host (code/TrimCDP-WB/src/GSTnonHop.cu:355-404,
 // code/PrunedDP++/include/CPUNONHOP.h:266-383 and :564-586).
+// Then the rest bounds: a tree that covers the groups of X contains a path between
+// members of any two of them, so it costs at least their largest group distance; doubled
+// it is a closed walk through every group of X, so it costs at least half of the cheapest
+// closed sequence min_{i,j} P[X][i][j] + vv[j][i].
 __device__ void build_tour(Ctx* c) {
   const int k = c->k, W = c->W;
   uint32_t* P = c->tour;
@@ -1570,6 +1588,18 @@ __device__ void build_tour(Ctx* c) {
       for (int p = 0; p < k; p++)
         if ((X >> p) & 1u) m = min(m, P[(size_t)X * TOUR_STRIDE + i * KMAX + p]);
     P2[(size_t)X * KMAX + i] = m;
+  }
+  uint32_t* R = P2 + (size_t)W * KMAX;
+  for (int X = threadIdx.x; X < W; X += blockDim.x) {
+    uint32_t far = 0;
+    uint64_t walk = COST_INF;
+    for (int i = 0; i < k; i++)
+      for (int j = 0; j < k; j++)
+        if (i != j && ((X >> i) & 1) && ((X >> j) & 1)) {
+          far = max(far, c->vv[i * KMAX + j]);
+          walk = min(walk, (uint64_t)P[(size_t)X * TOUR_STRIDE + i * KMAX + j] + c->vv[j * KMAX + i]);
+        }
+    R[X] = __popc(X) < 2 ? 0u : max(far, (uint32_t)((walk + 1) / 2));
   }
 }
 

@@ -70,7 +70,7 @@ struct SlotMem {
   uint32_t rowcap = 0, outcap = 0, stackcap = 0;
 };
 
-constexpr size_t kTourWords = ((size_t)1 << KMAX) * (TOUR_STRIDE + KMAX);
+constexpr size_t kTourWords = ((size_t)1 << KMAX) * (TOUR_STRIDE + KMAX + 1);
 constexpr uint32_t kOutCap = 1u << 16;
 constexpr uint32_t kStackCap = 1u << 18;
 
