@@ -101,10 +101,15 @@ enum ErrBits : uint32_t { ERR_QCAP = 1, ERR_FARCAP = 2, ERR_ROWCAP = 4, ERR_TIME
 constexpr uint32_t ROW_NONE = 0xFFFFFFFFu;
 enum CtrlMode : int { CTRL_SSSP = 0, CTRL_DP_ROWS = 1, CTRL_DP_GROW = 2 };
 
-// Light-edge index: per vertex, the number of edges of weight <= widx_threshold(t)
+// Light-edge index: per vertex, the number of edges of weight <= widx_threshold(t) << wsh
 // for t < WIDX, thresholds 1, 2, 3, 4, 6, 8, 12, ..., 192, 256 (each step x1.5 or
 // x1.33), so that one load bounds the edges a relaxation under a weight limit
-// needs, over-counting by at most a third.
+// needs, over-counting by at most a third.  The graph's shift wsh puts the thresholds
+// where its weights are: the smallest with 256 << wsh >= twice the median weight (0 up
+// to a median of 128; a few heavy outliers do not move it).  With weights of 1..10^6
+// (wsh = 12), where unscaled thresholds made every relaxation read the whole list,
+// 12 queries over 141k vertices relax 125 M edges without the shift and 25 M with it
+// (grow 4.6 to 3.1 ms, the call 15.2 to 13.6 ms).
 constexpr int WIDX = 16;
 constexpr uint32_t CHUNK = 0x80000000u;  // item flag (in pd): one `split`-edge chunk only
 constexpr int RELAX_U = 4;               // edges per lane per round of the grow relax loop
@@ -120,8 +125,9 @@ struct DevGraph {
   const int64_t* beg;     // V+1
   const int2* edges;      // E x {neighbour, weight}, sorted by neighbour per vertex
   const int2* wedges;     // the same edges sorted by (weight, neighbour) per vertex
-  const uint32_t* widx;   // V x WIDX: edges of v with weight <= 2^j (NULL: no index,
+  const uint32_t* widx;   // V x WIDX: edges of v up to each threshold (NULL: no index,
                           // wedges then need not be weight-sorted)
+  uint32_t wsh;           // the thresholds' shift
 };
 
 __host__ __device__ __forceinline__ uint32_t widx_threshold(int t) {
@@ -143,7 +149,7 @@ __device__ __forceinline__ int64_t count_upto(const DevGraph& G, uint32_t v, int
                                               uint32_t W) {
   if (deg <= 0 || W == 0u) return 0;
   if (!G.widx) return deg;
-  const int t = widx_slot(W);
+  const int t = widx_slot((W >> G.wsh) + ((W & ((1u << G.wsh) - 1u)) ? 1u : 0u));
   return t >= WIDX ? deg : (int64_t)__ldg(&G.widx[(uint64_t)v * WIDX + t]);
 }
 

@@ -178,6 +178,7 @@ struct gst_graph {
   int2* d_edges = nullptr;   // per vertex sorted by neighbour (tree extraction)
   int2* d_wedges = nullptr;  // per vertex sorted by (weight, neighbour) (grow, SSSP)
   uint32_t* d_widx = nullptr;
+  uint32_t wsh = 0;          // shift of the light-edge index's thresholds
   int64_t max_deg = 0;       // shape of the graph (autotuner cache key)
   int32_t max_w = 0;
   // Vertices are renumbered on the device by degree, highest first (ties by id), so that
@@ -280,7 +281,7 @@ gst_status status_of(const Ctx& c) {
 }
 
 DevGraph dev_graph(const gst_graph* g) {
-  return DevGraph{g->V, g->E, g->d_beg, g->d_edges, g->d_wedges, g->d_widx};
+  return DevGraph{g->V, g->E, g->d_beg, g->d_edges, g->d_wedges, g->d_widx, g->wsh};
 }
 
 // Grid of the rows kernel: every SM filled with as many CTAs as its registers and
@@ -1531,8 +1532,16 @@ static gst_status graph_create_impl(gst_engine* eng, int64_t V, int64_t E, const
   wt = nwt.data();
   // Two device copies of the adjacency: sorted by neighbour (edge-weight lookups
   // of the tree walk) and sorted by weight, with per vertex the number of edges of
-  // weight <= widx_threshold(t) (t < WIDX), so that a grow step reads only the edges light enough
-  // to keep its target under the upper bound.
+  // weight <= widx_threshold(t) << wsh (t < WIDX), so that a grow step reads only the edges
+  // light enough to keep its target under the upper bound.
+  uint32_t wsh = 0;
+  if (E > 0) {
+    std::vector<int32_t> some;  // the median of a sample spread over the edge list
+    for (int64_t i = 0, step = std::max<int64_t>(1, E / 65536); i < E; i += step) some.push_back(wt[i]);
+    std::nth_element(some.begin(), some.begin() + (std::ptrdiff_t)(some.size() / 2), some.end());
+    const int64_t reach = 2ll * some[some.size() / 2];
+    while (wsh < 16 && (256ll << wsh) < reach) wsh++;
+  }
   std::vector<int2> edges((size_t)E), wedges((size_t)E);
   std::vector<uint32_t> widx((size_t)V * WIDX);
   int bad = 0;
@@ -1554,7 +1563,7 @@ static gst_status graph_create_impl(gst_engine* eng, int64_t V, int64_t E, const
       std::sort(tmp.begin(), tmp.end());
       size_t j = 0;
       for (int t = 0; t < WIDX; t++) {
-        while (j < tmp.size() && (uint32_t)tmp[j].first <= widx_threshold(t)) j++;
+        while (j < tmp.size() && (uint32_t)tmp[j].first <= (widx_threshold(t) << wsh)) j++;
         widx[(size_t)v * WIDX + t] = (uint32_t)j;
       }
       for (size_t i = 0; i < tmp.size(); i++)
@@ -1569,6 +1578,7 @@ static gst_status graph_create_impl(gst_engine* eng, int64_t V, int64_t E, const
   g->eng = eng;
   g->V = V;
   g->E = E;
+  g->wsh = wsh;
   g->to_dev.swap(to_dev);
   g->to_host.swap(to_host);
   for (int64_t v = 0; v < V; v++) g->max_deg = std::max(g->max_deg, beg[v + 1] - beg[v]);
@@ -2564,7 +2574,7 @@ gst_status noalloc_solve(int device, cudaStream_t st, int64_t V, int64_t E, cons
   if (nhb) NCK(cudaMemsetAsync(c.dist_h, 0xFF, (size_t)nhb * Vs * ds * 4, st));
   NCK(cudaMemcpyAsync(d_ctx, &c, sizeof(Ctx), cudaMemcpyHostToDevice, st));
   // the caller's edges are sorted by neighbour only: no light-edge index
-  DevGraph G{V, E, d_beg, (const int2*)d_edges, (const int2*)d_edges, nullptr};
+  DevGraph G{V, E, d_beg, (const int2*)d_edges, (const int2*)d_edges, nullptr, 0u};
   k_init<<<dim3(64, 1), 256, 0, st>>>(d_ctx, 1, G, d_grp_ptr, d_members, split);
   k_ctrl<<<1, 32, 0, st>>>(d_ctx, 1, CTRL_SSSP);
   const size_t smem = rows_smem_per_warp((int)RW) * (size_t)warps;

@@ -40,7 +40,7 @@ def test_rest_bounds_never_exceed_the_optimum(hop, wmax):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("k,hop", [(1, None), (2, None), (2, 3), (5, 2), (7, None), (7, 3), (8, None)])
-@pytest.mark.parametrize("wmax", [2, 100, 1 << 20])
+@pytest.mark.parametrize("wmax", [2, 100, 1 << 20, 1 << 24])
 def test_engine_keeps_the_optimum(engine, k, hop, wmax):
     g = G.synth_rmat(700, 3000, 90 + k, wmax=wmax)
     grp = G.synth_groups_uniform(g.V, 30, 1, 40, 91)
