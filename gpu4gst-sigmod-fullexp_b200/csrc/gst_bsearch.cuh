@@ -12,7 +12,7 @@
 //
 // Cutoffs: a query's distances are needed exactly only up to its search cutoff (its star
 // bound x cut_pm / 1000).  Column c keeps the largest cutoff of the queries that use it;
-// stars are found while the search runs (before each relax step, k_bs_star sums each
+// stars are found while the search runs (before each relax step, k_bs_scan sums each
 // query's columns at every announced vertex) and the cutoffs only decrease, so every distance at
 // most a column's final cutoff is exact (every prefix of its shortest path stayed below
 // it) and every other one is only known to exceed it.  A query then takes the smallest
@@ -30,27 +30,49 @@
 // diameter <= D), as in the per-query search; after the last round the tables above
 // it are filled from it.
 //
-// Per step: k_bs_scan turns the announcement bits of the previous step into relax items
-// of at most BS_CHUNK edges (a hub's range spread over many warps), k_bs_star finds the
-// stars at the announced vertices and k_bs_ctrl lowers the cutoffs, k_bs_relax relaxes
-// the items, and k_bs_ctrl updates the cutoffs again and ends the search when nothing
-// was announced.
+// Edge classes (unbounded searches): the edges are relaxed light ones first, to a fixpoint,
+// and only then the heavier ones, from every vertex whose distances changed since its
+// heavier edges were last relaxed.  A relaxation is bound by the random row it reads, and
+// label-correcting steps over all edges repeat most of them: a vertex improves a few
+// columns at a time, step after step, and its heavy edges run before the cutoffs are
+// known.  The light fixpoint is a small share of the edges, settles nearly every distance
+// and finds the stars, so a heavy edge is relaxed about once, for all columns of a sector
+// together, against nearly final cutoffs.  Any order ends at the same distances.  On 32
+// queries of k = 5/7 over 141k vertices 464 M sectors are relaxed instead of 1013 M (search
+// 8.4 to 6.5 ms), on the 4M-vertex batch 5.3 G instead of 7.6 G (82 to 70 ms).  The light
+// steps are more and smaller, so a search over few columns or edges runs in one class: a
+// lone query takes 6.5 ms in one class and 8.9 ms in two at 4M vertices
+// (Runner::search_classes).
+//
+// Per step, two launches: k_bs_scan turns the announcement bits of the step's class into
+// relax items of at most BS_CHUNK edges (a hub's range spread over many warps) and finds
+// the stars at the announced vertices, its last block lowers the cutoffs; k_bs_relax
+// relaxes the items, its last block chooses the next step's class or ends the search.
 #pragma once
 #include "gst_device.cuh"
 
 namespace gst {
 
 constexpr int BS_COLS = 256;   // columns (distinct groups) of one shared search, at most
-constexpr int BS_CHUNK = 128;  // edges per relax item
 constexpr int BS_MAXQ = MAXB;  // queries of one shared search, at most
 
 struct BsCtx {
   uint32_t* dist;       // V x Gp distances, row v at dist + v * Gp
   uint32_t* fm[2];      // V x Wm announcement words (bit c: column c improved at v)
+  uint32_t* later;      // V x Wm, two classes: columns whose heavy edges wait
+  uint32_t ncls;        // edge classes: 1, or 2 (light edges, heavy edges)
+  const uint32_t* cend; // V, two classes: the end of v's light edges in its list
+  uint32_t cls;         // class of the current step
+  uint32_t have;        // later is not empty
+  uint32_t arrived;     // blocks of the current launch that are done (see last_block)
   uint32_t* am;         // V x Wm: v's active columns in the current step (scan -> relax)
-  uint2* items;         // relax items of the current step: {v, chunk}
+  uint2* items;         // relax items of the current step: {v, chunk}; whole chunks from the
+                        // front, the lists' ends (shorter ones) from the back
   uint32_t item_cap;
-  uint32_t n_items;     // items of the current step (appended by the scan)
+  uint32_t chunk;       // edges per item, at most
+  uint32_t n_items[2];  // whole and short items of the current step (appended by the scan)
+  unsigned long long work[2];  // their (edge, active sector) pairs
+  uint32_t next[2];     // items of each taken from the counter in the relax step
   uint32_t Gp, Wm;      // columns (a multiple of 8), mask words per vertex
   uint32_t in;          // fm[in] is scanned this step; fm[in ^ 1] takes its announcements
   uint32_t ann;         // the relax step announced something
@@ -68,6 +90,29 @@ struct BsCtx {
 };
 constexpr uint32_t BS_ERR_ITEMS = 1, BS_ERR_STEPS = 2;
 
+// True in the last block of the grid to get here, which then sees the other blocks'
+// writes; no block waits.  All threads of every block call it once per launch.
+__device__ __forceinline__ bool last_block(uint32_t* arrived) {
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(arrived, 1u) == gridDim.x - 1u;
+    if (s_last) *arrived = 0u;
+  }
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last;
+}
+
+// First and one-past-last edge of v's weight-sorted list in the current class.
+__device__ __forceinline__ void class_range(const BsCtx* b, uint32_t cls, uint32_t v, int64_t deg,
+                                            int64_t* lo, int64_t* hi) {
+  const int64_t light = b->ncls > 1u ? (int64_t)__ldg(&b->cend[v]) : deg;
+  *lo = cls ? light : 0;
+  *hi = cls ? deg : light;
+}
+
 // Seeds: column c's members at distance 0, announced (blockIdx.y = column).
 __global__ void k_bs_seed(BsCtx* b, DevGraph G, const int64_t* grp_ptr, const int32_t* members,
                           const int32_t* col_gid, int ncols) {
@@ -84,201 +129,424 @@ __global__ void k_bs_seed(BsCtx* b, DevGraph G, const int64_t* grp_ptr, const in
   }
 }
 
-// Scan: every vertex announced in the previous step gets its active columns (moved from
-// fm[in] to am) and one relax item per BS_CHUNK edges of its list.
-__global__ void k_bs_scan(BsCtx* b, DevGraph G) {
+// Column cutoffs from the query stars (the last block of a scan).
+__device__ __forceinline__ void bs_lower_cutoffs(BsCtx* b, uint32_t* s_cut) {
+  for (uint32_t c = threadIdx.x; c < BS_COLS; c += blockDim.x) s_cut[c] = 0u;
+  __syncthreads();
+  for (uint32_t x = threadIdx.x; x < b->nq * KMAX; x += blockDim.x) {
+    const uint32_t q = x / KMAX, i = x % KMAX;
+    if (i >= b->qk[q]) continue;
+    const uint32_t st = __ldcg(&b->star[q]);
+    const uint64_t cut = st == COST_INF ? COST_INF : (uint64_t)st * b->cut_pm / 1000u;
+    // a used column's cutoff is stored plus one, below: 0 marks an unused column
+    atomicMax(&s_cut[b->qcol[q][i]], cut >= COST_INF ? COST_INF : (uint32_t)cut + 1u);
+  }
+  __syncthreads();
+  for (uint32_t c = threadIdx.x; c < b->Gp; c += blockDim.x)
+    if (s_cut[c] && s_cut[c] != COST_INF) b->cutc[c] = min(b->cutc[c], s_cut[c] - 1u);
+}
+
+// Scan: every vertex announced for the step's class gets its active columns (moved to am,
+// and on to the next class's waiting columns) and its relax items: one per chunk of the
+// edges it has in the class.  Then its stars: each query's columns summed at the vertex
+// (the query's k shortest paths from there form a connected subgraph covering every group,
+// a feasible cost); hop-bounded from table r with 2r <= D only (a tree of diameter <= D).
+// A star found here lowers the cutoffs that this very step relaxes against.  One lane per
+// (vertex, query).  VPT neighbouring vertices per thread: with four, their words come in
+// Wm 16-byte loads issued together, which is all a step that announces few vertices does
+// (large graphs); with one, the stars of a small graph spread over four times the warps.
+template <int VPT>
+__global__ void __launch_bounds__(256) k_bs_scan(BsCtx* b, DevGraph G) {
+  __shared__ uint32_t s_star[BS_MAXQ];
+  __shared__ uint32_t s_cut[BS_COLS];
+  __shared__ uint16_t s_col[BS_MAXQ][KMAX];
+  __shared__ uint32_t s_k[BS_MAXQ];
+  __shared__ uint32_t s_v[256 / 32][32];  // per warp: the announced vertices
+  __shared__ uint32_t s_sum[2][256 / 32], s_work[2][256 / 32], s_base[2];
   if (b->done) return;
-  const uint32_t Wm = b->Wm;
-  uint32_t* fi = b->fm[b->in];
-  const int lane = threadIdx.x & 31;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < G.V;
+  const uint32_t Wm = b->Wm, cls = b->cls, Gp = b->Gp, nq = b->nq, D = b->D, r = b->round;
+  const uint32_t chunk = b->chunk, cap = b->item_cap;
+  uint32_t* from = cls ? b->later : b->fm[b->in];
+  uint32_t* later = cls + 1u < b->ncls ? b->later : nullptr;
+  // Every improved distance is announced to the light class, and on to the heavy one.  With
+  // two classes the light scans, of which there are many, look for stars only at the
+  // vertices of highest degree (the lowest ids), where the best ones are, and the heavy
+  // scans everywhere: star passes in all of them took a third of the relax steps' time.
+  const bool stars = D == 0u || (r >= 1u && 2u * r <= D);
+  const int64_t star_end = !D && cls == 0u && b->ncls > 1u ? (G.V + 15) / 16 : G.V;
+  const uint32_t* tab = D ? b->tab[r] : b->dist;
+  for (uint32_t q = threadIdx.x; q < BS_MAXQ; q += blockDim.x) {
+    s_star[q] = COST_INF;
+    s_k[q] = q < nq ? b->qk[q] : 0u;
+#pragma unroll
+    for (int i = 0; i < KMAX; i++) s_col[q][i] = q < nq ? b->qcol[q][i] : 0u;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  uint32_t more = 0;
+  const int64_t spans = (G.V + VPT - 1) / VPT;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < spans;
        base += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t v = base + threadIdx.x;
-    uint32_t nchunks = 0;
-    if (v < G.V) {
-      uint32_t x[BS_COLS / 32];
-      uint32_t any = 0;
-#pragma unroll
-      for (uint32_t w = 0; w < BS_COLS / 32; w++) {
-        x[w] = w < Wm ? __ldcg(&fi[(uint64_t)v * Wm + w]) : 0u;
-        any |= x[w];
-      }
-      if (any) {
-        // the announcements become this step's active columns; the words are cleared
-        // for the step after next
-#pragma unroll
-        for (uint32_t w = 0; w < BS_COLS / 32; w++)
-          if (w < Wm) {
-            b->am[(uint64_t)v * Wm + w] = x[w];
-            fi[(uint64_t)v * Wm + w] = 0u;
-          }
-        const int64_t deg = G.beg[v + 1] - G.beg[v];
-        nchunks = (uint32_t)((deg + BS_CHUNK - 1) / BS_CHUNK);
+    const int64_t first = (base + threadIdx.x) * VPT;
+    uint32_t hit = 0;  // bit i: vertex first + i is announced
+    if (base + threadIdx.x < spans) {
+      if (VPT == 4) {
+        const uint4* p = (const uint4*)(from + first * Wm);
+        for (uint32_t w = 0; w < Wm; w++) {  // its word 4 w + i is vertex first + (4 w + i) / Wm's
+          const uint4 x = p[w];  // (a cached load: a line serves several of them)
+          hit |= (x.x ? 1u << (4 * w) / Wm : 0u) | (x.y ? 1u << (4 * w + 1) / Wm : 0u) |
+                 (x.z ? 1u << (4 * w + 2) / Wm : 0u) | (x.w ? 1u << (4 * w + 3) / Wm : 0u);
+        }
+      } else {
+        for (uint32_t w = 0; w < Wm; w++) hit |= __ldcg(&from[first * Wm + w]) ? 1u : 0u;
       }
     }
-    // warp-aggregated reservation of the items
-    const uint32_t scan = warp_incl_scan(nchunks);
-    const uint32_t tot = __shfl_sync(0xffffffffu, scan, 31);
-    uint32_t basei = 0;
-    if (lane == 31 && tot) basei = atomicAdd(&b->n_items, tot);
-    basei = __shfl_sync(0xffffffffu, basei, 31);
-    for (uint32_t j = 0; j < nchunks; j++) {
-      const uint32_t i = basei + scan - nchunks + j;
-      if (i < b->item_cap) b->items[i] = make_uint2((uint32_t)v, j);
-      else atomicOr(&b->error, BS_ERR_ITEMS);
+    if (!__syncthreads_or(hit != 0u)) continue;
+    uint32_t whole[VPT], rest[VPT], nw = 0, nr = 0, ww = 0, wr = 0;
+#pragma unroll
+    for (int i = 0; i < VPT; i++) {
+      whole[i] = rest[i] = 0u;
+      if (!((hit >> i) & 1u)) continue;
+      const uint32_t v = (uint32_t)(first + i);
+      uint32_t sectors = 0;
+      for (uint32_t w = 0; w < Wm; w++) {
+        const uint32_t x = __ldcg(&from[(uint64_t)v * Wm + w]);
+        b->am[(uint64_t)v * Wm + w] = x;
+        from[(uint64_t)v * Wm + w] = 0u;
+        if (later && x) later[(uint64_t)v * Wm + w] |= x;
+        sectors += ((x & 0xFFu) != 0u) + ((x & 0xFF00u) != 0u) + ((x & 0xFF0000u) != 0u) + (x >> 24 != 0u);
+      }
+      more |= later != nullptr;
+      int64_t lo, hi;
+      class_range(b, cls, v, G.beg[v + 1] - G.beg[v], &lo, &hi);
+      const uint32_t edges = (uint32_t)(hi - lo);
+      whole[i] = edges / chunk;
+      rest[i] = edges % chunk != 0u;
+      nw += whole[i];
+      nr += rest[i];
+      ww += whole[i] * sectors;
+      wr += edges % chunk * sectors;
     }
+    // one reservation per block and list: a per-warp one made the counters the hottest
+    // address of the step
+    const uint32_t sw = warp_incl_scan(nw), sr = warp_incl_scan(nr);
+    ww = __reduce_add_sync(0xffffffffu, ww);
+    wr = __reduce_add_sync(0xffffffffu, wr);
+    if (lane == 31) {
+      s_sum[0][wib] = sw;
+      s_sum[1][wib] = sr;
+      s_work[0][wib] = ww;
+      s_work[1][wib] = wr;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+      uint32_t tot = 0;
+      unsigned long long work = 0;
+      for (uint32_t w = 0; w < blockDim.x / 32; w++) {
+        const uint32_t x = s_sum[threadIdx.x][w];
+        s_sum[threadIdx.x][w] = tot;
+        tot += x;
+        work += (unsigned long long)s_work[threadIdx.x][w] * (threadIdx.x == 0 ? chunk : 1u);
+      }
+      s_base[threadIdx.x] = tot ? atomicAdd(&b->n_items[threadIdx.x], tot) : 0u;
+      if (work) atomicAdd(&b->work[threadIdx.x], work);
+    }
+    __syncthreads();
+    uint32_t tw = s_base[0] + s_sum[0][wib] + sw - nw, tr = s_base[1] + s_sum[1][wib] + sr - nr;
+    if (tw + nw + tr + nr > cap) atomicOr(&b->error, BS_ERR_ITEMS);
+#pragma unroll
+    for (int i = 0; i < VPT; i++) {
+      // a hub's items (hundreds) are written by the whole warp
+      uint32_t hubs = __ballot_sync(0xffffffffu, whole[i] > 16u);
+      while (hubs) {
+        const int src = __ffs(hubs) - 1;
+        hubs &= hubs - 1u;
+        const uint32_t n = __shfl_sync(0xffffffffu, whole[i], src), t = __shfl_sync(0xffffffffu, tw, src);
+        const uint32_t v = __shfl_sync(0xffffffffu, (uint32_t)(first + i), src);
+        for (uint32_t j = (uint32_t)lane; j < n; j += 32)
+          if (t + j < cap) b->items[t + j] = make_uint2(v, j);
+      }
+      if (whole[i] <= 16u)
+        for (uint32_t j = 0; j < whole[i]; j++)
+          if (tw + j < cap) b->items[tw + j] = make_uint2((uint32_t)(first + i), j);
+      tw += whole[i];
+      if (rest[i]) {
+        if (tr < cap) b->items[cap - 1u - tr] = make_uint2((uint32_t)(first + i), whole[i]);
+        tr++;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < VPT; i++) {
+      const uint32_t ann = __ballot_sync(0xffffffffu, (hit >> i) & 1u);
+      if (!stars || !ann || (base + (threadIdx.x & ~31u)) * VPT >= star_end) continue;
+      if ((hit >> i) & 1u) s_v[wib][__popc(ann & ((1u << lane) - 1u))] = (uint32_t)(first + i);
+      __syncwarp();
+      for (uint32_t p = (uint32_t)lane; p < __popc(ann) * nq; p += 32) {
+        const uint32_t a = nq == 1u ? p : p / nq, q = p - a * nq, k = s_k[q];
+        const uint32_t* row = tab + (uint64_t)s_v[wib][a] * Gp;
+        uint64_t sum = 0;
+#pragma unroll
+        for (uint32_t t = 0; t < KMAX; t++) sum += t < k ? row[s_col[q][t]] : 0u;
+        if (sum < (uint64_t)s_star[q]) atomicMin(&s_star[q], (uint32_t)sum);
+      }
+      __syncwarp();
+    }
+  }
+  if (__any_sync(0xffffffffu, more != 0u) && lane == 0) b->have = 1u;
+  __syncthreads();
+  for (uint32_t q = threadIdx.x; q < nq; q += blockDim.x)
+    if (s_star[q] < __ldcg(&b->star[q])) atomicMin(&b->star[q], s_star[q]);
+  if (!last_block(&b->arrived)) return;
+  if (stars) bs_lower_cutoffs(b, s_cut);
+  if (threadIdx.x == 0 && cls) b->have = 0u;  // this scan took them all
+}
+
+// The next step (the last block of a relax launch): announced vertices first, else the
+// heavy edges that wait; without any the search is done.
+__device__ __forceinline__ void bs_advance(BsCtx* b) {
+  const uint32_t cls = __ldcg(&b->ann) ? 0u : 1u;
+  if (__ldcg(&b->error) || (cls && !__ldcg(&b->have))) {
+    b->done = 1u;
+  } else if (++b->steps > b->max_steps) {
+    b->error |= BS_ERR_STEPS;
+    b->done = 1u;
+  } else {
+    b->cls = cls;
+    if (cls == 0u) b->in ^= 1u;
+    b->ann = 0u;
+    for (int i = 0; i < 2; i++) {
+      b->n_items[i] = b->next[i] = 0u;
+      b->work[i] = 0ull;
+    }
+    b->round++;
   }
 }
 
-// Relax: one item per warp iteration, in two phases.  First lane s holds sector s
-// (columns 8s..8s+7) of the item's vertex: its distances, active bits and, per active
-// column, the heaviest edge it may still take (`lim`).  Then the work is the
-// item's edges times its nA sectors with an active column, spread over all 32 lanes:
-// lane t takes active sector t mod nA and the edges t / nA, t / nA + R, ... (R = 32 /
-// nA), reading that sector of each target's row, relaxing and announcing the improved
-// columns.  The kernel is bound by instruction issue, not memory (a row is one
-// contiguous span), and an item rarely has more than a few active sectors, so the
-// edge loop is what the compaction keeps busy.
+// Relax.  A warp takes up to 32 items at a time and lists their units, the (item, active
+// 8-column sector) pairs; 32 units form a window.  Lane t loads the distances of unit t's
+// sector, stages them in shared memory and plans the item's edges (those light enough for
+// some of its columns).  Then the window's work, every (edge, sector) pair of its items, is
+// spread over all lanes: item by item, edge by edge, the sectors of one edge on neighbouring
+// lanes, so that a target's row is read as one contiguous span.  One item per warp left most
+// of it idle in the light classes, whose items have a few edges each behind a chain of
+// dependent loads; fixed shares of the items left most warps waiting for the few that held
+// the hubs, so the warps take items from a counter, the whole chunks
+// first.  In one class, against one item per warp in fixed shares: 23 to 9 ms of relax steps
+// for three lone queries over 4M vertices, 3.9 to 2.7 ms over 141k; 77 to 74 ms for the
+// 4M-vertex batch, whose items are wide (57 ms with the two classes).  Two pairs per lane
+// and four blocks per SM: three pairs in 80 registers and three blocks take 10 % longer on
+// the batches, five blocks spill.
+// The test of a sector is two instructions per column: with the sector's -d and cutoff + 1,
+// some column improves over the edge's weight w iff max_i(min(target_i, cutoff_i + 1) - d_i) > w.
+constexpr int BS_U = 2;        // (edge, sector) pairs per lane in flight
+constexpr uint32_t BS_TAKE = 1024;  // pairs per take, about
+constexpr uint32_t BS_LIST = 256;   // units per take, at most
+struct __align__(16) BsUnit {  // one unit of a window
+  int nd[8];                   // -distance per column (inactive: -INT_MAX)
+  uint32_t sec;                // the sector
+  uint32_t pad[3];             // 48-byte stride: eight lanes' 16-byte loads hit 32 banks
+};
+struct __align__(16) BsWork {  // one item of a window with work
+  int64_t eb;                  // its first edge
+  uint32_t start;              // its first pair in the window
+  uint32_t unit;               // its first unit | its units c << 5 | ceil(2^16 / c) << 11: a
+                               // pair's edge is (pair * that) >> 16, exact below 2^11 pairs
+};
 __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G) {
-  __shared__ uint32_t s_cut[BS_COLS];
-  __shared__ uint16_t s_split[33][32];           // [nA][t]: t mod nA | (t / nA) << 8
-  __shared__ unsigned char s_map[256 / 32][32];  // per warp: active index -> sector
+  // (shared memory is kept small: what it leaves to the L1 serves the edge lists)
+  __shared__ __align__(16) int s_c1[BS_COLS / 8][12];  // per sector and column: cutoff + 1
+  __shared__ BsUnit s_unit[256 / 32][32];              // per warp: the window's units
+  __shared__ BsWork s_work[256 / 32][32];              // per warp: the window's items
+  __shared__ uint16_t s_list[256 / 32][BS_LIST];       // per warp: lane of the item << 5 | sector
   if (b->done) return;
   const uint32_t Gp = b->Gp, Wm = b->Wm, nsec = Gp / 8u;
-  for (uint32_t c = threadIdx.x; c < BS_COLS; c += blockDim.x) s_cut[c] = c < Gp ? b->cutc[c] : 0u;
-  for (uint32_t x = threadIdx.x; x < 33u * 32u; x += blockDim.x) {
-    const uint32_t na = x >> 5, t = x & 31u;
-    s_split[na][t] = na ? (uint16_t)((t % na) | ((t / na) << 8)) : 0;
-  }
+  for (uint32_t c = threadIdx.x; c < BS_COLS; c += blockDim.x)
+    s_c1[c >> 3][c & 7u] = c < Gp ? (int)(min(b->cutc[c], 0x7FFFFFFEu) + 1u) : 0;
   __syncthreads();
   // hop-bounded round r: sources in table r (the members at 0 for r = 0), targets in
   // table r + 1; a round's paths extend only while they have fewer than D edges
-  const uint32_t D = b->D, r = b->round;
-  if (D && r >= D) return;
-  const uint32_t* src_tab = D ? (r ? b->tab[r] : nullptr) : b->dist;
-  uint32_t* dst_tab = D ? b->tab[r + 1] : b->dist;
+  const uint32_t D = b->D, r = b->round, cls = b->cls, chunk_edges = b->chunk, cap = b->item_cap;
+  const bool over = (D && r >= D) || b->error;  // past the last round: nothing to relax
+  const uint32_t* src_tab = D ? (r ? b->tab[min(r, D)] : nullptr) : b->dist;
+  uint32_t* dst_tab = D ? b->tab[min(r + 1u, D)] : b->dist;
   const bool extend = D == 0u || r + 1u < D;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const uint32_t n = min(b->n_items, b->item_cap);
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  // neighbouring takes go to different blocks: the first ones hold the hubs' chunks
+  const uint32_t wid = (uint32_t)wib * gridDim.x + blockIdx.x;
   uint32_t* fo = b->fm[b->in ^ 1u];
-  const bool mine = (uint32_t)lane < nsec;
-  const uint32_t s = (uint32_t)lane;
   unsigned long long relaxed = 0;
   uint32_t any = 0;
-  for (uint32_t it = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < n; it += warps) {
-    const uint2 item = b->items[it];
-    const uint32_t v = item.x, chunk = item.y;
-    uint32_t m = 0;
-    if (mine) m = (__ldcg(&b->am[(uint64_t)v * Wm + (s >> 2)]) >> ((s & 3u) * 8u)) & 0xFFu;
-    uint32_t dv[8];
+  for (int kind = 0; kind < 2 && !over; kind++) {
+   const uint32_t n = b->n_items[kind];
+   // about BS_TAKE pairs, and no more than spreads the step over all warps
+   const uint32_t per = n ? (uint32_t)((unsigned long long)BS_TAKE * n / max(b->work[kind], 1ull)) : 0u;
+   const uint32_t take =
+       max(1u, min(min(min(32u, BS_LIST / nsec), per), (n + warps - 1u) / warps));
+   // A warp's first take is its own share where the step is small (no contention for the
+   // counter when most warps have nothing to do); else all come from the counter, so that
+   // no share waits for a warp that is still at work on the whole chunks.
+   const bool shares = kind ? n <= warps * take && b->n_items[0] <= warps / 8u : true;
+   const uint32_t taken = shares ? warps * take : 0u;
+   uint32_t base = wid * take;
+   if (!shares) {
+     if (lane == 0) base = atomicAdd(&b->next[kind], take);
+     base = __shfl_sync(0xffffffffu, base, 0);
+   }
+   while (base < n) {
+    // the items' active sectors, listed in item order
+    uint2 item = make_uint2(0u, 0u);
+    uint32_t sectors = 0;
+    if ((uint32_t)lane < take && base + lane < n) {
+      item = b->items[kind ? cap - 1u - (base + lane) : base + lane];
+      for (uint32_t w = 0; w < Wm; w++) {
+        const uint32_t x = __ldcg(&b->am[(uint64_t)item.x * Wm + w]);
 #pragma unroll
-    for (int i = 0; i < 8; i++) dv[i] = COST_INF;
-    if (mine && !src_tab) {
-#pragma unroll
-      for (int i = 0; i < 8; i++)
-        if ((m >> i) & 1u) dv[i] = 0u;  // round 0: the members themselves
-    } else if (mine && m) {
-      const uint4* src = (const uint4*)&src_tab[(uint64_t)v * Gp + s * 8];
-      const uint4 a = __ldcg(src), c4 = __ldcg(src + 1);
-      dv[0] = a.x;
-      dv[1] = a.y;
-      dv[2] = a.z;
-      dv[3] = a.w;
-      dv[4] = c4.x;
-      dv[5] = c4.y;
-      dv[6] = c4.z;
-      dv[7] = c4.w;
+        for (int j = 0; j < 4; j++)
+          if ((x >> (8 * j)) & 0xFFu) sectors |= 1u << (4 * w + j);
+      }
     }
-    // per active column: the heaviest edge it may still take from v (0: none; edge
-    // weights are at least 1), and for the warp the heaviest of them all
-    uint32_t lim[8], wl = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      const uint32_t cut = mine ? s_cut[s * 8 + i] : 0u;
-      lim[i] = (((m >> i) & 1u) && dv[i] < cut) ? cut - dv[i] : 0u;
-      wl = max(wl, lim[i]);
-    }
-    const uint32_t amask = __ballot_sync(0xffffffffu, wl != 0u);
-    wl = __reduce_max_sync(0xffffffffu, wl);
-    if (!amask) continue;
-    const int64_t b0 = G.beg[v], b1 = G.beg[v + 1];
-    const int64_t cnt = count_upto(G, v, b1 - b0, wl);
-    const int64_t e0 = (int64_t)chunk * BS_CHUNK, e1 = min(cnt, e0 + BS_CHUNK);
-    if (e1 <= e0) continue;
-    // work: the target-row sectors this item reads, one per active sector and edge
-    const uint32_t nA = (uint32_t)__popc(amask);
-    relaxed += (unsigned long long)(e1 - e0) * nA;
-    // compaction: active index -> sector, then each lane takes its sector's values
-    if ((amask >> lane) & 1u) s_map[wib][__popc(amask & ((1u << lane) - 1u))] = (unsigned char)lane;
+    const uint32_t uscan = warp_incl_scan((uint32_t)__popc(sectors));
+    const uint32_t units = __shfl_sync(0xffffffffu, uscan, 31);
+    uint32_t at = uscan - (uint32_t)__popc(sectors);
+    for (uint32_t m = sectors; m; m &= m - 1u) s_list[wib][at++] = (uint16_t)(lane << 5 | (__ffs(m) - 1));
     __syncwarp();
-    const uint32_t sp = s_split[nA][lane];
-    const uint32_t R = 32u / nA;  // edges per round (warp-uniform)
-    const uint32_t sec = s_map[wib][sp & 0xFFu];
-    const int64_t joff = (int64_t)(sp >> 8);
-    uint32_t dx[8], lx[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-      dx[i] = __shfl_sync(0xffffffffu, dv[i], (int)sec);
-      lx[i] = __shfl_sync(0xffffffffu, lim[i], (int)sec);
-    }
-    if (joff >= (int64_t)R) continue;  // lanes beyond R x nA
-    int64_t e = e0 + joff;
-    // the edges are sorted by weight: a lane stops at the first one heavier than every
-    // limit of its sector; two edges per lane in flight
-    uint32_t lmax = 0;
-#pragma unroll
-    for (int i = 0; i < 8; i++) lmax = max(lmax, lx[i]);
-    const int64_t R2 = 2 * (int64_t)R;
-    int2 ea = e < e1 ? G.wedges[b0 + e] : make_int2(0, 0);
-    int2 eb = e + R < e1 ? G.wedges[b0 + e + R] : make_int2(0, 0);
-    for (; e < e1; e += R2) {
-      const bool hb = e + R < e1;
-      const uint32_t ua = (uint32_t)ea.x, wa = (uint32_t)ea.y;
-      const uint32_t ub = (uint32_t)eb.x, wb = (uint32_t)eb.y;
-      if (wa > lmax) break;
-      const bool ga = ua < G.V, gb = hb && wb <= lmax && ub < G.V;
-      uint4 ra0 = make_uint4(0, 0, 0, 0), ra1 = ra0, rb0 = ra0, rb1 = ra0;
-      if (ga) {
-        const uint4* dst = (const uint4*)&dst_tab[(uint64_t)ua * Gp + sec * 8];
-        ra0 = __ldcg(dst);
-        ra1 = __ldcg(dst + 1);
+    for (uint32_t u0 = 0; u0 < units; u0 += 32) {
+      const uint32_t live = min(32u, units - u0);
+      const uint32_t ent = s_list[wib][u0 + min((uint32_t)lane, live - 1u)];
+      const uint32_t sec = ent & 31u, own = ent >> 5;
+      const uint32_t v = __shfl_sync(0xffffffffu, item.x, (int)own);
+      const uint32_t chunk = __shfl_sync(0xffffffffu, item.y, (int)own);
+      const uint32_t m = (__ldcg(&b->am[(uint64_t)v * Wm + (sec >> 2)]) >> ((sec & 3u) * 8u)) & 0xFFu;
+      uint4 da = make_uint4(0, 0, 0, 0), db = da;  // round 0: the members themselves
+      if (src_tab) {
+        const uint4* src = (const uint4*)&src_tab[(uint64_t)v * Gp + sec * 8];
+        da = __ldcg(src);
+        db = __ldcg(src + 1);
       }
-      if (gb) {
-        const uint4* dst = (const uint4*)&dst_tab[(uint64_t)ub * Gp + sec * 8];
-        rb0 = __ldcg(dst);
-        rb1 = __ldcg(dst + 1);
+      const int64_t b0 = G.beg[v], b1 = G.beg[v + 1];
+      int64_t lo, hi;
+      class_range(b, cls, v, b1 - b0, &lo, &hi);
+      const uint32_t dv[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+      BsUnit x;
+      int wl = 0;  // heaviest edge some column of the unit may still take
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        const int c1 = s_c1[sec][i];
+        const bool on = ((m >> i) & 1u) && dv[i] < (uint32_t)c1 - 1u;
+        x.nd[i] = on ? -(int)dv[i] : -0x7FFFFFFF;
+        wl = max(wl, c1 + x.nd[i] - 1);
       }
-      if (e + R2 < e1) ea = G.wedges[b0 + e + R2];
-      if (e + R2 + R < e1) eb = G.wedges[b0 + e + R2 + R];
+      x.sec = sec;
+      s_unit[wib][lane] = x;
+      // the units of one item are neighbours: `lead` its first lane in the window, `cnt`
+      // their number; the item's edges up to the largest limit among them
+      uint32_t cnt = 1;
+      bool lead = (uint32_t)lane < live;
+      if (Gp > 8u) {
+        const uint32_t prev = __shfl_up_sync(0xffffffffu, own, 1);
+        lead = lead && (lane == 0 || prev != own);
+        const uint32_t heads = __ballot_sync(0xffffffffu, lead);
+        const uint32_t above = lane == 31 ? 0u : heads >> (lane + 1);
+        const uint32_t end = above ? (uint32_t)(lane + __ffs(above)) : live;
+        cnt = end > (uint32_t)lane ? end - lane : 0u;
 #pragma unroll
-      for (int x = 0; x < 2; x++) {
-        const bool g = x ? gb : ga;
-        const uint32_t u = x ? ub : ua, w = x ? wb : wa;
-        const uint4 r0 = x ? rb0 : ra0, r1 = x ? rb1 : ra1;
-        if (!g) continue;
-        const uint32_t du[8] = {r0.x, r0.y, r0.z, r0.w, r1.x, r1.y, r1.z, r1.w};
-        uint32_t imp = 0;
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_down_sync(0xffffffffu, wl, o);
+          if ((uint32_t)(lane + o) < end) wl = max(wl, y);
+        }
+      }
+      int64_t eb = 0;
+      uint32_t work = 0;
+      if (lead && wl > 0) {
+        const int64_t e0 = lo + (int64_t)chunk * chunk_edges;
+        const int64_t e1 = min(min(hi, count_upto(G, v, b1 - b0, (uint32_t)wl)), e0 + chunk_edges);
+        if (e1 > e0) work = (uint32_t)(e1 - e0) * cnt;
+        eb = b0 + e0;
+      }
+      const uint32_t scan = warp_incl_scan(work);
+      const uint32_t tot = __shfl_sync(0xffffffffu, scan, 31);
+      const uint32_t start = scan - work;
+      // the items with work, in order; a pair's item follows from the starts below it
+      const uint32_t busy = __ballot_sync(0xffffffffu, work != 0u);
+      if (work) s_work[wib][__popc(busy & ((1u << lane) - 1u))] = BsWork{eb, start, (uint32_t)lane | cnt << 5 | ((0xFFFFu + cnt) / cnt) << 11};
+      relaxed += tot;
+      __syncwarp();
+      const uint32_t mark = work ? start : 0xFFFFFFFFu;
+      uint32_t before = 0;  // items that start before this round's pairs
+      for (uint32_t j0 = 0; j0 < tot; j0 += 32 * BS_U) {
+        uint32_t tu[BS_U], un[BS_U], at[BS_U];
+        int tw[BS_U];
+        uint4 ra[BS_U], rb[BS_U];
+        bool ok[BS_U];
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          if (w <= lx[i]) {
-            const uint32_t nd = dx[i] + w;
-            if (nd < du[i]) {
-              atomicMin(&dst_tab[(uint64_t)u * Gp + sec * 8 + i], nd);
-              if (w < lx[i] && extend) imp |= 1u << i;
-            }
+        for (int y = 0; y < BS_U; y++) {
+          const uint32_t jb = j0 + (uint32_t)y * 32u, j = jb + lane;
+          const uint32_t starts = __reduce_or_sync(0xffffffffu, mark - jb < 32u ? 1u << (mark - jb) : 0u);
+          const uint32_t o = before + __popc(starts & (0xFFFFFFFFu >> (31 - lane))) - 1u;
+          before += __popc(starts);
+          const BsWork q = s_work[wib][o];
+          ok[y] = j < tot;
+          const uint32_t loc = ok[y] ? j - q.start : 0u;
+          uint32_t e = loc, su = 0;
+          if (Gp > 8u) {
+            e = (loc * (q.unit >> 11)) >> 16;
+            su = loc - e * ((q.unit >> 5) & 63u);
+          }
+          un[y] = (q.unit & 31u) + su;
+          const int2 ed = ok[y] ? G.wedges[q.eb + e] : make_int2(0, 0);
+          tu[y] = (uint32_t)ed.x;
+          tw[y] = ed.y;
+          ok[y] = ok[y] && tu[y] < G.V;
+        }
+#pragma unroll
+        for (int y = 0; y < BS_U; y++) {
+          at[y] = tu[y] * nsec + s_unit[wib][un[y]].sec;
+          ra[y] = rb[y] = make_uint4(0, 0, 0, 0);
+          if (ok[y]) {
+            ra[y] = __ldcg((const uint4*)(dst_tab + (uint64_t)at[y] * 8u));
+            rb[y] = __ldcg((const uint4*)(dst_tab + (uint64_t)at[y] * 8u) + 1);
           }
         }
-        if (imp) {
-          atomicOr(&fo[(uint64_t)u * Wm + (sec >> 2)], imp << ((sec & 3u) * 8u));
-          any = 1u;
+#pragma unroll
+        for (int y = 0; y < BS_U; y++) {
+          if (!ok[y]) continue;
+          const BsUnit& q = s_unit[wib][un[y]];
+          const int* c1 = s_c1[q.sec];
+          const int w = tw[y];
+          const uint32_t du[8] = {ra[y].x, ra[y].y, ra[y].z, ra[y].w, rb[y].x, rb[y].y, rb[y].z, rb[y].w};
+          int best = -0x7FFFFFFF;
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            best = __viaddmax_s32((int)min(du[i], (uint32_t)c1[i]), q.nd[i], best);
+          if (best <= w) continue;
+          uint32_t imp = 0, ann = 0;
+#pragma unroll
+          for (int i = 0; i < 8; i++)
+            imp |= (int)min(du[i], (uint32_t)c1[i]) + q.nd[i] > w ? 1u << i : 0u;
+          for (; imp; imp &= imp - 1u) {
+            const int i = __ffs(imp) - 1;
+            const int nd = w - q.nd[i];
+            atomicMin(dst_tab + (uint64_t)at[y] * 8u + i, (uint32_t)nd);
+            if (extend && nd + 1 < c1[i]) ann |= 1u << i;
+          }
+          if (ann) {
+            const uint32_t col = q.sec * 8u;
+            atomicOr(&fo[(uint64_t)tu[y] * Wm + (col >> 5)], ann << (col & 31u));
+            any = 1u;
+          }
         }
       }
+      __syncwarp();
     }
+    if (lane == 0) base = taken + atomicAdd(&b->next[kind], take);
+    base = __shfl_sync(0xffffffffu, base, 0);
+   }
   }
   any = __reduce_or_sync(0xffffffffu, any);
   if (lane == 0 && any) b->ann = 1u;
   if (lane == 0 && relaxed) atomicAdd(&b->st_relax, relaxed);  // the same in every lane
+  if (last_block(&b->arrived) && threadIdx.x == 0) bs_advance(b);
 }
 
 // Hop-bounded tables (n4 = V x Gp / 4 uint4 per table).  Before round r >= 1:
@@ -303,95 +571,6 @@ __global__ void k_bs_copy(BsCtx* b, int64_t n4, int finish) {
        i += (int64_t)gridDim.x * blockDim.x) {
     const uint4 x = __ldcs(src + i);
     for (uint32_t h = from + 1u; h <= h1; h++) __stcs((uint4*)b->tab[h] + i, x);
-  }
-}
-
-// Stars, before the relax step: at every vertex announced for this step (the first
-// chunk of its items), each query's columns summed (the query's k shortest paths from v
-// form a connected subgraph covering every group, a feasible cost).  Hop-bounded: from
-// table r with 2r <= D only (a tree of diameter <= D).  Found before the relax step, a
-// star lowers the cutoffs that this very step relaxes against.
-__global__ void __launch_bounds__(256) k_bs_star(BsCtx* b) {
-  __shared__ __align__(16) uint32_t s_row[256 / 32][BS_COLS];  // per warp: the vertex's row
-  __shared__ uint32_t s_star[BS_MAXQ];
-  if (b->done) return;
-  const uint32_t D = b->D, r = b->round;
-  if (D && !(r >= 1u && 2u * r <= D)) return;
-  const uint32_t* src_tab = D ? b->tab[r] : b->dist;
-  const uint32_t Gp = b->Gp, nsec = Gp / 8u, nq = b->nq;
-  for (uint32_t q = threadIdx.x; q < BS_MAXQ; q += blockDim.x) s_star[q] = COST_INF;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const uint32_t n = min(b->n_items, b->item_cap);
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  for (uint32_t base = wid * 32u; base < n; base += warps * 32u) {
-    // lane i looks at item base + i; the warp then takes the first chunks one by one
-    uint32_t v = 0;
-    bool first = false;
-    if (base + lane < n) {
-      const uint2 item = b->items[base + lane];
-      v = item.x;
-      first = item.y == 0u;
-    }
-    uint32_t todo = __ballot_sync(0xffffffffu, first);
-    while (todo) {
-      const int src = __ffs(todo) - 1;
-      todo &= todo - 1u;
-      const uint32_t x = __shfl_sync(0xffffffffu, v, src);
-      if ((uint32_t)lane < nsec) {
-        const uint4* p = (const uint4*)&src_tab[(uint64_t)x * Gp + lane * 8];
-        const uint4 a = __ldcg(p), c4 = __ldcg(p + 1);
-        uint4* o = (uint4*)&s_row[wib][lane * 8];
-        o[0] = a;
-        o[1] = c4;
-      }
-      __syncwarp();
-      for (uint32_t q = (uint32_t)lane; q < nq; q += 32) {
-        uint64_t sum = 0;
-        for (uint32_t i = 0; i < b->qk[q]; i++) sum += s_row[wib][b->qcol[q][i]];
-        if (sum < (uint64_t)s_star[q]) atomicMin(&s_star[q], (uint32_t)sum);
-      }
-      __syncwarp();
-    }
-  }
-  __syncthreads();
-  for (uint32_t q = threadIdx.x; q < nq; q += blockDim.x)
-    if (s_star[q] < COST_INF) atomicMin(&b->star[q], s_star[q]);
-}
-
-// Control (one block): column cutoffs from the query stars; with `advance`, after the
-// relax step, the next step's buffers and the end of the search.
-__global__ void k_bs_ctrl(BsCtx* b, int advance) {
-  if (b->done) return;
-  const uint32_t nq = b->nq, Gp = b->Gp;
-  for (uint32_t c = threadIdx.x; c < Gp; c += blockDim.x) {
-    uint32_t mx = 0;
-    bool used = false;
-    for (uint32_t q = 0; q < nq; q++)
-      for (uint32_t i = 0; i < b->qk[q]; i++)
-        if (b->qcol[q][i] == c) {
-          used = true;
-          const uint32_t st = b->star[q];
-          const uint64_t x = st == COST_INF ? COST_INF : (uint64_t)st * b->cut_pm / 1000u;
-          mx = max(mx, x >= COST_INF ? COST_INF : (uint32_t)x);
-        }
-    if (used) b->cutc[c] = min(b->cutc[c], mx);
-  }
-  if (!advance) return;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (b->error || !b->ann) {
-      b->done = 1u;
-    } else if (++b->steps > b->max_steps) {
-      b->error |= BS_ERR_STEPS;
-      b->done = 1u;
-    } else {
-      b->ann = 0u;
-      b->in ^= 1u;
-      b->n_items = 0u;
-      b->round++;
-    }
   }
 }
 

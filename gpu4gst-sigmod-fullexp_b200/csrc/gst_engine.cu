@@ -179,6 +179,8 @@ struct gst_graph {
   int2* d_wedges = nullptr;  // per vertex sorted by (weight, neighbour) (grow, SSSP)
   uint32_t* d_widx = nullptr;
   uint32_t wsh = 0;          // shift of the light-edge index's thresholds
+  uint32_t* d_cend = nullptr;  // where each vertex's light edges end in its weight-sorted
+                               // list (the shared distance search's edge classes)
   int64_t max_deg = 0;       // shape of the graph (autotuner cache key)
   int32_t max_w = 0;
   // Vertices are renumbered on the device by degree, highest first (ties by id), so that
@@ -796,6 +798,16 @@ struct Runner {
     }
   }
 
+  // Edge classes of an unbounded shared search over ncols columns (gst_bsearch.cuh).  Two
+  // pay from about 5e8 (edge, 8-column sector) pairs on, or 1.5e8 when the rows are wide:
+  // 22 and 22 ms (one class, two) at 5.6e8 pairs of 4M vertices, 38 and 31 at 1.1e9; with
+  // 15 sectors 17.4 and 16.6 at 4.4e8 pairs of 1M, 5.1 and 4.3 at 1.8e8 of 141k; but 8.6
+  // and 10.4 at 2.4e8 pairs of 1M in 8 sectors, 14 and 16 at 2.8e8 of 4M in 2.
+  int search_classes(uint32_t ncols) const {
+    const double sectors = (ncols + 7u) / 8u, pairs = sectors * (double)g->E;
+    return pairs >= 5e8 || (sectors >= 12 && pairs >= 1.5e8) ? 2 : 1;
+  }
+
   // One batch-shared distance search for the queries `jobs`, all unbounded (D = 0) or all
   // of hop bound D (1..KMAX), over their distinct groups `cols` (at most BS_COLS groups,
   // BS_MAXQ queries).  On success every job is marked (ss = 1) with its columns and
@@ -806,8 +818,11 @@ struct Runner {
     const uint32_t ncols = (uint32_t)cols.size();
     const uint32_t Gp = (ncols + 7u) / 8u * 8u, Wm = (Gp + 31u) / 32u;
     if (D < 0 || D > KMAX) return GST_OK;
-    const uint64_t item_cap = (uint64_t)V + (uint64_t)g->E / BS_CHUNK + 1024;
-    if (item_cap >= (1ull << 32)) return GST_OK;
+    // edges per relax item: fewer the wider the rows, so that an item is a share of a step
+    const uint32_t chunk = Gp <= 32 ? 128 : Gp <= 96 ? 64 : 32;
+    const uint64_t item_cap = (uint64_t)V + (uint64_t)g->E / chunk + 1024;
+    // 32-bit item and sector indexes
+    if (item_cap >= (1ull << 32) || (uint64_t)V * (Gp / 8) >= (1ull << 32)) return GST_OK;
     size_t off = 0;
     auto take = [&](size_t n) {
       const size_t o = off;
@@ -816,9 +831,12 @@ struct Runner {
     };
     const size_t o_b = take(sizeof(BsCtx));
     const size_t o_dist = take((size_t)V * Gp * 4 * (size_t)std::max(D, 1));  // tables 1..D
-    const size_t o_fm0 = take((size_t)V * Wm * 4);
-    const size_t o_fm1 = take((size_t)V * Wm * 4);
-    const size_t o_am = take((size_t)V * Wm * 4);
+    const size_t words = ((size_t)V + 3) / 4 * 16 * Wm;  // whole quads of vertices (k_bs_scan)
+    const size_t o_fm0 = take(words);
+    const size_t o_fm1 = take(words);
+    const size_t o_am = take(words);
+    const int ncls = D ? 1 : search_classes(ncols);
+    const size_t o_later = take(ncls > 1 ? words : 0);
     const size_t o_items = take((size_t)item_cap * 8);
     const size_t o_cols = take((size_t)BS_COLS * 4);
     void* p = nullptr;
@@ -839,8 +857,12 @@ struct Runner {
     h.fm[0] = (uint32_t*)(base + o_fm0);
     h.fm[1] = (uint32_t*)(base + o_fm1);
     h.am = (uint32_t*)(base + o_am);
+    h.ncls = (uint32_t)ncls;
+    h.later = ncls > 1 ? (uint32_t*)(base + o_later) : nullptr;
+    h.cend = g->d_cend;
     h.items = (uint2*)(base + o_items);
     h.item_cap = (uint32_t)item_cap;
+    h.chunk = chunk;
     h.Gp = Gp;
     h.Wm = Wm;
     h.max_steps = (uint32_t)std::min(eng->cfg.max_levels, 1 << 16);
@@ -868,8 +890,9 @@ struct Runner {
     CK(cudaEventRecord(eng->bs_ev[0], st));
     // the seeds' table (table 1 of a hop-bounded search); the copies fill the others
     CK(cudaMemsetAsync(D ? h.tab[1] : h.dist, 0xFF, (size_t)V * Gp * 4, st));
-    CK(cudaMemsetAsync(h.fm[0], 0, (size_t)V * Wm * 4, st));
-    CK(cudaMemsetAsync(h.fm[1], 0, (size_t)V * Wm * 4, st));
+    CK(cudaMemsetAsync(h.fm[0], 0, words, st));
+    CK(cudaMemsetAsync(h.fm[1], 0, words, st));
+    if (ncls > 1) CK(cudaMemsetAsync(h.later, 0, words, st));
     CK(cudaMemcpyAsync(d_b, &h, sizeof(BsCtx), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_cols, cols.data(), ncols * 4, cudaMemcpyHostToDevice, st));
     cs.h2d += sizeof(BsCtx) + ncols * 4;
@@ -880,6 +903,8 @@ struct Runner {
     int occ = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bs_relax, 256, 0);
     const int relax_blocks = eng->sms * std::max(1, std::min(occ, 4));
+    const bool wide = V >= 600000;  // four vertices per scan thread
+    const int scan_blocks = (int)std::min<int64_t>(eng->sms * 8, wide ? (V + 1023) / 1024 : (V + 255) / 256);
     BsCtx hb;
     for (;;) {
       for (int i = 0; i < 6; i++) {
@@ -887,15 +912,13 @@ struct Runner {
           k_bs_copy<<<eng->sms * 4, 256, 0, st>>>(d_b, n4, 0);
           launches++;
         }
-        k_bs_scan<<<eng->sms * 4, 256, 0, st>>>(d_b, G);
-        k_bs_star<<<eng->sms * 4, 256, 0, st>>>(d_b);
-        k_bs_ctrl<<<1, 256, 0, st>>>(d_b, 0);
+        if (wide) k_bs_scan<4><<<scan_blocks, 256, 0, st>>>(d_b, G);
+        else k_bs_scan<1><<<scan_blocks, 256, 0, st>>>(d_b, G);
         const int pe = prof_begin(PROF_BSRELAX);
         k_bs_relax<<<relax_blocks, 256, 0, st>>>(d_b, G);
         prof_end(pe);
         relax_launches++;
-        k_bs_ctrl<<<1, 256, 0, st>>>(d_b, 1);
-        launches += 5;
+        launches += 2;
       }
       CK(cudaGetLastError());
       CK(cudaMemcpyAsync(&hb, d_b, sizeof(BsCtx), cudaMemcpyDeviceToHost, st));
@@ -1572,6 +1595,18 @@ static gst_status graph_create_impl(gst_engine* eng, int64_t V, int64_t E, const
   }
   if (bad & 1) return fail(eng, GST_BAD_INPUT, "graph: neighbour id out of range");
   if (bad & 2) return fail(eng, GST_BAD_INPUT, "graph: weights must be in [1, 2^24]");
+  // The light edges of the shared distance search: the index slot that holds nearest to an
+  // eighth of all edges.
+  std::vector<uint32_t> cend((size_t)V);
+  {
+    double share[WIDX] = {};
+    for (int64_t v = 0; v < V; v++)
+      for (int t = 0; t < WIDX; t++) share[t] += widx[(size_t)v * WIDX + t];
+    int best = 0;
+    for (int t = 1; t < WIDX; t++)
+      if (std::abs(share[t] - (double)E / 8) < std::abs(share[best] - (double)E / 8)) best = t;
+    for (int64_t v = 0; v < V; v++) cend[(size_t)v] = widx[(size_t)v * WIDX + best];
+  }
   std::lock_guard<std::mutex> lk(eng->mu);
   CK(cudaSetDevice(eng->device));
   gst_graph* g = new gst_graph();
@@ -1587,6 +1622,7 @@ static gst_status graph_create_impl(gst_engine* eng, int64_t V, int64_t E, const
   CK(cudaMalloc(&g->d_edges, sizeof(int2) * std::max<int64_t>(E, 1)));
   CK(cudaMalloc(&g->d_wedges, sizeof(int2) * std::max<int64_t>(E, 1)));
   CK(cudaMalloc(&g->d_widx, sizeof(uint32_t) * V * WIDX));
+  CK(cudaMalloc(&g->d_cend, sizeof(uint32_t) * V));
   // stream-ordered copies, completed before returning: the level kernels run on a
   // non-blocking stream that does not wait for the legacy default stream
   CK(cudaMemcpyAsync(g->d_beg, beg, sizeof(int64_t) * (V + 1), cudaMemcpyHostToDevice,
@@ -1599,6 +1635,8 @@ static gst_status graph_create_impl(gst_engine* eng, int64_t V, int64_t E, const
   }
   CK(cudaMemcpyAsync(g->d_widx, widx.data(), sizeof(uint32_t) * V * WIDX,
                      cudaMemcpyHostToDevice, eng->stream));
+  CK(cudaMemcpyAsync(g->d_cend, cend.data(), sizeof(uint32_t) * V, cudaMemcpyHostToDevice,
+                     eng->stream));
   CK(cudaStreamSynchronize(eng->stream));
   eng->graphs++;
   *out = g;
@@ -1635,6 +1673,7 @@ gst_status gst_graph_destroy(gst_graph* g) {
   cudaFree(g->d_edges);
   cudaFree(g->d_wedges);
   cudaFree(g->d_widx);
+  cudaFree(g->d_cend);
   cudaMemPoolTrimTo(eng->pool, 0);
   delete g;
   eng->graphs--;
