@@ -626,11 +626,14 @@ __global__ void k_gather_dist(uint32_t* rows, uint32_t ds, int k, GroupVecs gv, 
 }
 
 // ---- init: group members -> zero-cost singletons, SSSP sources, dirty rows ----
+// One group per blockIdx.z (KMAX of them): its members' dependent accesses (row map, pool,
+// cell, row list) run beside the other groups' instead of after them.
 __global__ void k_init(Ctx* ctxs, int nctx, DevGraph G, const int64_t* grp_ptr,
                        const int32_t* members, int split) {
   for (int qi = blockIdx.y; qi < nctx; qi += gridDim.y) {
     Ctx* c = ctxs + qi;
-    for (int i = 0; i < c->k; i++) {
+    const int i = (int)blockIdx.z;
+    if (i < c->k) {
       const int32_t g = c->gid[i];
       const int64_t b = grp_ptr[g], e = grp_ptr[g + 1];
       for (int64_t j = b + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < e;
@@ -1558,42 +1561,49 @@ __device__ __forceinline__ void ctrl_take_far(Ctx* c) {
 // members of any two of them, so it costs at least their largest group distance; doubled
 // it is a closed walk through every group of X, so it costs at least half of the cheapest
 // closed sequence min_{i,j} P[X][i][j] + vv[j][i].
-__device__ void build_tour(Ctx* c) {
+// One entry P[X][i][p] per thread and round, the rounds by the size of X.  The table is
+// built in the block's dynamic shared memory (`P`, W x TOUR_STRIDE words) where the launch
+// has it and copied out, else in place: its chain of dependent reads took 146 us for k = 7
+// and 23 us for k = 5 in global memory with one (X, i) per thread; now 24 and 10 us.
+__device__ void build_tour(Ctx* c, uint32_t* P) {
+  __shared__ uint32_t vv[KMAX * KMAX];
   const int k = c->k, W = c->W;
-  uint32_t* P = c->tour;
+  const bool in_place = P == c->tour;
+  for (int i = threadIdx.x; i < KMAX * KMAX; i += blockDim.x) vv[i] = c->vv[i];
+  __syncthreads();
   for (int L = 1; L <= k; L++) {
-    for (int idx = threadIdx.x; idx < W * k; idx += blockDim.x) {
-      const uint32_t X = (uint32_t)(idx / k);
-      const int i = idx - (int)X * k;
-      if (__popc(X) != L || !((X >> i) & 1u)) continue;
-      for (int p = 0; p < k; p++) {
-        if (!((X >> p) & 1u)) continue;
-        uint32_t val = COST_INF;
-        if (L == 1) {
-          val = 0u;  // X == {i}, p == i
-        } else if (p != i) {
-          const uint32_t prev = X ^ (1u << p);
-          for (int j = 0; j < k; j++) {
-            if (!((prev >> j) & 1u)) continue;
-            const uint64_t x = (uint64_t)P[(size_t)prev * TOUR_STRIDE + i * KMAX + j] +
-                               c->vv[j * KMAX + p];
+    for (int idx = threadIdx.x; idx < W * TOUR_STRIDE; idx += blockDim.x) {
+      const uint32_t X = (uint32_t)idx / TOUR_STRIDE;
+      const int i = (idx / KMAX) % KMAX, p = idx % KMAX;
+      if (__popc(X) != L || !((X >> i) & 1u) || !((X >> p) & 1u)) continue;
+      uint32_t val = COST_INF;
+      if (L == 1) {
+        val = 0u;  // X == {i}, p == i
+      } else if (p != i) {
+        const uint32_t prev = X ^ (1u << p);
+        const uint32_t* from = P + prev * TOUR_STRIDE + i * KMAX;
+#pragma unroll
+        for (int j = 0; j < KMAX; j++)
+          if ((prev >> j) & 1u) {
+            const uint64_t x = (uint64_t)from[j] + vv[j * KMAX + p];
             if (x < val) val = (uint32_t)x;
           }
-        }
-        P[(size_t)X * TOUR_STRIDE + i * KMAX + p] = val;
       }
+      P[idx] = val;
     }
     __syncthreads();
   }
-  uint32_t* P2 = P + (size_t)W * TOUR_STRIDE;
-  for (int idx = threadIdx.x; idx < W * k; idx += blockDim.x) {
-    const uint32_t X = (uint32_t)(idx / k);
-    const int i = idx - (int)X * k;
+  if (!in_place)
+    for (int idx = threadIdx.x; idx < W * TOUR_STRIDE; idx += blockDim.x) c->tour[idx] = P[idx];
+  uint32_t* P2 = c->tour + (size_t)W * TOUR_STRIDE;
+  for (int idx = threadIdx.x; idx < W * KMAX; idx += blockDim.x) {
+    const uint32_t X = (uint32_t)(idx / KMAX);
+    const int i = idx % KMAX;
     uint32_t m = COST_INF;
     if ((X >> i) & 1u)
       for (int p = 0; p < k; p++)
-        if ((X >> p) & 1u) m = min(m, P[(size_t)X * TOUR_STRIDE + i * KMAX + p]);
-    P2[(size_t)X * KMAX + i] = m;
+        if ((X >> p) & 1u) m = min(m, P[X * TOUR_STRIDE + i * KMAX + p]);
+    P2[idx] = m;
   }
   uint32_t* R = P2 + (size_t)W * KMAX;
   for (int X = threadIdx.x; X < W; X += blockDim.x) {
@@ -1602,8 +1612,8 @@ __device__ void build_tour(Ctx* c) {
     for (int i = 0; i < k; i++)
       for (int j = 0; j < k; j++)
         if (i != j && ((X >> i) & 1) && ((X >> j) & 1)) {
-          far = max(far, c->vv[i * KMAX + j]);
-          walk = min(walk, (uint64_t)P[(size_t)X * TOUR_STRIDE + i * KMAX + j] + c->vv[j * KMAX + i]);
+          far = max(far, vv[i * KMAX + j]);
+          walk = min(walk, (uint64_t)P[X * TOUR_STRIDE + i * KMAX + j] + vv[j * KMAX + i]);
         }
     R[X] = __popc(X) < 2 ? 0u : max(far, (uint32_t)((walk + 1) / 2));
   }
@@ -1621,8 +1631,10 @@ __device__ __forceinline__ void ctrl_start_dp(Ctx* c) {
 }
 
 // One block per query context; thread 0 runs the control logic, the whole block
-// builds the tour table when a query leaves its distance phase.
-__global__ void k_ctrl(Ctx* ctxs, int nctx, int mode) {
+// builds the tour table when a query leaves its distance phase (in `shared` bytes of
+// dynamic shared memory where they hold it).
+__global__ void __launch_bounds__(512) k_ctrl(Ctx* ctxs, int nctx, int mode, int shared) {
+  extern __shared__ uint32_t s_tour[];
   const int qi = blockIdx.x;
   if (qi >= nctx) return;
   Ctx* c = ctxs + qi;
@@ -1642,7 +1654,8 @@ __global__ void k_ctrl(Ctx* ctxs, int nctx, int mode) {
     const uint32_t lim = cut == COST_INF ? COST_INF : cut + 1u;
     for (int i = threadIdx.x; i < KMAX * KMAX; i += blockDim.x) c->vv[i] = min(c->vv[i], lim);
     __syncthreads();
-    if (c->use_tour) build_tour(c);  // block-uniform branch
+    if (c->use_tour)  // block-uniform branch
+      build_tour(c, shared >= c->W * TOUR_STRIDE * 4 ? s_tour : c->tour);
     if (threadIdx.x == 0) {
       c->cut = cut;
       ctrl_start_dp(c);
@@ -1756,71 +1769,84 @@ __device__ int32_t edge_weight_dev(const DevGraph& G, uint32_t v, uint32_t u) {
   return w;
 }
 
+// One warp per query.  The states of the walk wait in a queue (`stack`: a walk has at most
+// one state per edge and two per merge, of which there are at most k - 1) and a lane
+// follows one each, so a round of dependent reads serves a whole generation of the tree;
+// the edges' weights are looked up at the end, one edge per lane.  One thread per query
+// took 168 us a walk (k = 5/7, 141k vertices), most of it in binary searches for weights,
+// now 19 us.
 __global__ void k_extract(Ctx* ctxs, int nctx, DevGraph G) {
-  const int qi = blockIdx.x * blockDim.x + threadIdx.x;
+  const int qi = blockIdx.x, lane = threadIdx.x;
   if (qi >= nctx) return;
   Ctx* c = ctxs + qi;
-  c->n_out = 0;
+  if (lane == 0) c->n_out = 0;
   if (c->phase != PH_DONE || c->best == ~0ull) return;
   const uint32_t v0 = (uint32_t)(c->best & 0x7FFFFFFull);
   const uint32_t d0 = (uint32_t)((c->best >> 27) & 31u);
   const uint64_t RW = (uint64_t)c->RW;
-  const uint32_t DD = (uint32_t)c->DD;
+  const uint32_t DD = (uint32_t)c->DD, cap = c->stackcap;
   const int k = c->k;
-  uint32_t sp = 0, nout = 0, steps = 0;
-  c->stack[sp++] = (uint64_t)v0 * RW + ((uint64_t)d0 << k) + (uint64_t)c->full;
-  while (sp > 0) {
-    if (++steps > 4u * c->stackcap) {
-      c->error |= ERR_EXTRACT;
+  uint32_t head = 0, tail = 1, nout = 0;
+  bool bad = false;
+  if (lane == 0) c->stack[0] = (uint64_t)v0 * RW + ((uint64_t)d0 << k) + (uint64_t)c->full;
+  __syncwarp();
+  while (head < tail) {
+    const uint32_t n = min(32u, tail - head);
+    uint64_t next[2];
+    uint32_t push = 0, u = 0, v = 0;
+    bool edge = false;
+    if ((uint32_t)lane < n) {
+      const uint64_t idx = c->stack[head + lane];
+      bad = !in_bounds(c, idx < (uint64_t)G.V * RW, 10);
+      v = bad ? 0u : (uint32_t)(idx / RW);
+      const uint32_t r = bad ? 0u : (uint32_t)(idx - (uint64_t)v * RW);
+      const uint32_t p = r & (uint32_t)c->full, d = r >> k;
+      const uint64_t* vrow = row_of(c, v);
+      const uint64_t cell = vrow ? vrow[r] : CELL_INF;
+      const uint32_t par = (uint32_t)cell & ~PEND;
+      if (cost_of(cell) == COST_INF) {  // a parent pointer never leads to an unreached state
+        bad = true;
+      } else if (par == LEAF) {
+        push = 0;
+      } else if (!(par & MERGE)) {
+        u = par;
+        bad = bad || u >= G.V || (c->hop && d == 0);
+        edge = true;
+        push = 1;
+        next[0] = (uint64_t)u * RW + ((uint64_t)(d - (uint32_t)c->hop) << k) + p;
+      } else {
+        const uint32_t Y = par & 0xFFFFu, d2 = (par >> 16) & 31u, d1 = (par >> 21) & 31u;
+        const uint32_t X = p ^ Y;
+        bad = bad || Y == 0 || (Y & ~p) != 0 || X == 0 || d1 >= DD || d2 >= DD;
+        push = 2;
+        next[0] = (uint64_t)v * RW + ((uint64_t)d1 << k) + X;
+        next[1] = (uint64_t)v * RW + ((uint64_t)d2 << k) + Y;
+      }
+    }
+    const uint32_t scan = warp_incl_scan(push);
+    const uint32_t total = __shfl_sync(0xffffffffu, scan, 31);
+    if (__any_sync(0xffffffffu, bad) || total > cap - tail) {
+      bad = true;
       break;
     }
-    const uint64_t idx = c->stack[--sp];
-    if (!in_bounds(c, idx < (uint64_t)G.V * RW, 10)) break;
-    const uint32_t v = (uint32_t)(idx / RW);
-    const uint32_t r = (uint32_t)(idx - (uint64_t)v * RW);
-    const uint32_t p = r & (uint32_t)c->full, d = r >> k;
-    const uint64_t* vrow = row_of(c, v);
-    const uint64_t cell = vrow ? vrow[r] : CELL_INF;
-    const uint32_t par = (uint32_t)cell & ~PEND;
-    if (cost_of(cell) == COST_INF) {  // a parent pointer never leads to an unreached state
-      c->error |= ERR_EXTRACT;
-      break;
+    for (uint32_t i = 0; i < push; i++) c->stack[tail + scan - push + i] = next[i];
+    const uint32_t edges = __ballot_sync(0xffffffffu, edge);
+    const uint32_t at = nout + (uint32_t)__popc(edges & ((1u << lane) - 1u));
+    if (edge && at < c->outcap) {
+      c->out[3 * at + 0] = (int32_t)u;
+      c->out[3 * at + 1] = (int32_t)v;
     }
-    if (par == LEAF) continue;
-    if (!(par & MERGE)) {
-      const uint32_t u = par;
-      if (u >= G.V || (c->hop && d == 0)) {
-        c->error |= ERR_EXTRACT;
-        break;
-      }
-      if (nout < c->outcap) {
-        c->out[3 * nout + 0] = (int32_t)u;
-        c->out[3 * nout + 1] = (int32_t)v;
-        c->out[3 * nout + 2] = edge_weight_dev(G, v, u);
-      }
-      nout++;
-      if (sp + 1 > c->stackcap) {
-        c->error |= ERR_EXTRACT;
-        break;
-      }
-      c->stack[sp++] = (uint64_t)u * RW + ((uint64_t)(d - (uint32_t)c->hop) << k) + p;
-    } else {
-      const uint32_t Y = par & 0xFFFFu, d2 = (par >> 16) & 31u, d1 = (par >> 21) & 31u;
-      const uint32_t X = p ^ Y;
-      if (Y == 0 || (Y & ~p) != 0 || X == 0 || d1 >= DD || d2 >= DD) {
-        c->error |= ERR_EXTRACT;
-        break;
-      }
-      if (sp + 2 > c->stackcap) {
-        c->error |= ERR_EXTRACT;
-        break;
-      }
-      c->stack[sp++] = (uint64_t)v * RW + ((uint64_t)d1 << k) + X;
-      c->stack[sp++] = (uint64_t)v * RW + ((uint64_t)d2 << k) + Y;
-    }
+    nout += (uint32_t)__popc(edges);
+    head += n;
+    tail += total;
+    __syncwarp();
   }
-  if (nout > c->outcap) c->error |= ERR_EXTRACT;
-  c->n_out = nout;
+  for (uint32_t i = (uint32_t)lane; i < min(nout, c->outcap); i += 32)
+    c->out[3 * i + 2] = edge_weight_dev(G, (uint32_t)c->out[3 * i + 1], (uint32_t)c->out[3 * i]);
+  if (lane == 0) {
+    if (bad || nout > c->outcap) c->error |= ERR_EXTRACT;
+    c->n_out = nout;
+  }
 }
 
 }  // namespace gst

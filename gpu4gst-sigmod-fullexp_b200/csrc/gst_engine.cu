@@ -768,7 +768,7 @@ struct Runner {
           cs.launches += 1;
         }
     }
-    k_init<<<dim3(64, 1), 256, 0, st>>>(d_ctx + s, 1, G, grp->d_ptr, grp->d_mem,
+    k_init<<<dim3(8, 1, KMAX), 256, 0, st>>>(d_ctx + s, 1, G, grp->d_ptr, grp->d_mem,
                                        eng->cfg.split_degree);
     if (n_cached == q->k || shared) {
       // the bounds pass over the distance rows (star bound, group distances), which
@@ -776,7 +776,8 @@ struct Runner {
       k_sssp<<<eng->sssp_blocks, 256, 0, st>>>(d_ctx + s, 1, G, eng->cfg.split_degree);
       cs.launches += 1;
     }
-    k_ctrl<<<1, 32, 0, st>>>(d_ctx + s, 1, CTRL_SSSP);
+    const int tour_bytes = c.W * TOUR_STRIDE * 4;
+    k_ctrl<<<1, 512, tour_bytes, st>>>(d_ctx + s, 1, CTRL_SSSP, tour_bytes);
     cs.launches += 2;
     owner[s] = j;
     idle_written[s] = 0;
@@ -1003,7 +1004,7 @@ struct Runner {
       const int pe = prof ? prof_begin(PROF_SSSP) : -1;
       k_sssp<<<eng->sssp_blocks, 256, 0, st>>>(d_ctx, nctx, G, split);
       prof_end(pe);
-      k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nctx, CTRL_SSSP);
+      k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nctx, CTRL_SSSP, 0);
     }
     const size_t per_warp = rows_smem_per_warp(rwm);
     // k_rows: at most 256 threads, as many warps as the widest row lets fit
@@ -1012,11 +1013,11 @@ struct Runner {
     k_rows<<<rows_blocks(eng, warps * 32, per_warp * warps), warps * 32, per_warp * warps, st>>>(
         d_ctx, nctx, G, split, rwm);
     prof_end(pe);
-    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nctx, CTRL_DP_ROWS);
+    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nctx, CTRL_DP_ROWS, 0);
     pe = prof ? prof_begin(PROF_GROW) : -1;
     k_grow<<<eng->grow_blocks, 256, 0, st>>>(d_ctx, nctx, G, split);
     prof_end(pe);
-    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nctx, CTRL_DP_GROW);
+    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nctx, CTRL_DP_GROW, 0);
   }
 
   // The level loop as a CUDA graph: a WHILE node whose body is one level plus a
@@ -1133,7 +1134,7 @@ struct Runner {
     for (int s = 0; s < nctx; s++) any |= owner[s] && h_ctx[s].phase >= PH_DONE;
     if (!any) return GST_OK;
     const DevGraph G = dev_graph(g);
-    k_extract<<<1, MAXB, 0, eng->stream>>>(d_ctx, nctx, G);
+    k_extract<<<nctx, 32, 0, eng->stream>>>(d_ctx, nctx, G);
     cs.launches += 1;
     CK(cudaMemcpyAsync(h_ctx, d_ctx, sizeof(Ctx) * nctx, cudaMemcpyDeviceToHost, eng->stream));
     cs.d2h += (int64_t)sizeof(Ctx) * nctx;
@@ -1479,11 +1480,13 @@ gst_status gst_engine_create(int32_t device, const gst_config* cfg, gst_engine**
   cudaMemPoolSetAttribute(eng->pool, cudaMemPoolAttrReleaseThreshold, &keep);
   eng->rows_smem = rows_smem_limit(device);
   if (cudaFuncSetAttribute(k_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)eng->rows_smem) != cudaSuccess) {
+                           (int)eng->rows_smem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_ctrl, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (1 << KMAX) * TOUR_STRIDE * 4) != cudaSuccess) {
     cudaStreamDestroy(eng->stream);
     cudaMemPoolDestroy(eng->pool);
     delete eng;
-    return fail(nullptr, GST_DEVICE_ERROR, "engine: cannot size the rows kernel's shared memory");
+    return fail(nullptr, GST_DEVICE_ERROR, "engine: cannot size the kernels' shared memory");
   }
   *out = eng;
   return GST_OK;
@@ -2614,19 +2617,19 @@ gst_status noalloc_solve(int device, cudaStream_t st, int64_t V, int64_t E, cons
   NCK(cudaMemcpyAsync(d_ctx, &c, sizeof(Ctx), cudaMemcpyHostToDevice, st));
   // the caller's edges are sorted by neighbour only: no light-edge index
   DevGraph G{V, E, d_beg, (const int2*)d_edges, (const int2*)d_edges, nullptr, 0u};
-  k_init<<<dim3(64, 1), 256, 0, st>>>(d_ctx, 1, G, d_grp_ptr, d_members, split);
-  k_ctrl<<<1, 32, 0, st>>>(d_ctx, 1, CTRL_SSSP);
+  k_init<<<dim3(8, 1, KMAX), 256, 0, st>>>(d_ctx, 1, G, d_grp_ptr, d_members, split);
+  k_ctrl<<<1, 32, 0, st>>>(d_ctx, 1, CTRL_SSSP, 0);
   const size_t smem = rows_smem_per_warp((int)RW) * (size_t)warps;
   int64_t launches = 2;
   Ctx h;
   for (;;) {
     for (int i = 0; i < 6; i++) {
       k_sssp<<<nd->sssp_blocks, 256, 0, st>>>(d_ctx, 1, G, split);
-      k_ctrl<<<1, 128, 0, st>>>(d_ctx, 1, CTRL_SSSP);
+      k_ctrl<<<1, 128, 0, st>>>(d_ctx, 1, CTRL_SSSP, 0);
       k_rows<<<nd->sms * 4, warps * 32, smem, st>>>(d_ctx, 1, G, split, (int)RW);
-      k_ctrl<<<1, 128, 0, st>>>(d_ctx, 1, CTRL_DP_ROWS);
+      k_ctrl<<<1, 128, 0, st>>>(d_ctx, 1, CTRL_DP_ROWS, 0);
       k_grow<<<nd->grow_blocks, 256, 0, st>>>(d_ctx, 1, G, split);
-      k_ctrl<<<1, 128, 0, st>>>(d_ctx, 1, CTRL_DP_GROW);
+      k_ctrl<<<1, 128, 0, st>>>(d_ctx, 1, CTRL_DP_GROW, 0);
       launches += 6;
     }
     NCK(cudaGetLastError());
