@@ -574,18 +574,4 @@ __global__ void k_bs_copy(BsCtx* b, int64_t n4, int finish) {
   }
 }
 
-// A query's distance rows (stride ds) from a shared table (V x Gp): column cols[i] for
-// group i.
-__global__ void k_bs_gather(uint32_t* rows, uint32_t ds, int k, const uint32_t* table, uint32_t Gp,
-                            ushort4 c0, ushort4 c1, int64_t V) {
-  const uint16_t cols[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V;
-       v += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t d[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++) d[i] = i < k ? __ldcg(&table[(uint64_t)v * Gp + cols[i]]) : COST_INF;
-    store_drow(rows, ds, (uint64_t)v, make_uint4(d[0], d[1], d[2], d[3]), make_uint4(d[4], d[5], d[6], d[7]));
-  }
-}
-
 }  // namespace gst

@@ -608,30 +608,112 @@ __device__ __forceinline__ void add_stat(Ctx* ctxs, int qi, bool valid, uint32_t
     atomicAdd(&(ctxs[qi].*field), (unsigned long long)tot);
 }
 
-// ---- group cache: distance rows of a query from cached per-group vectors ----------
-struct GroupVecs {
-  const uint32_t* v[KMAX];  // d_i(.) of the query's i-th group, V entries each (nullptr:
-                            // not cached, left unreached for the distance search)
+// ---- admission: the per-vertex buffers of queries that start together -----------------
+// One pass over the vertices for all of them: empty row maps, dirty bits and frontier
+// bytes, the state rows the slot's last query wrote, and the distance rows, gathered from
+// a shared search's tables or the group cache (or left unreached for the query's own
+// search).  Gathered distances are final, so the same pass takes what the bounds need of
+// them: the star bound min_v sum_i d_i(v) (the cost of the k shortest paths from the best
+// centre v, a feasible tree, so a valid ub), for a hop-bounded query also the best star of
+// D/2-edge paths (see k_sssp), and the group distances vv.  The queries of a batch read the
+// rows of one shared table, so a block takes them through its vertices one after another:
+// the row is read from memory once.  With up to twelve fills, gathers and passes per query
+// instead, starting 100 queries over 20k vertices took 3.5 ms more (call 12.7 to 10.2 ms),
+// 32 hop-bounded ones over 1M vertices 3 ms (32 to 28.7 ms).
+struct AdmitQ {
+  uint32_t slot;
+  uint32_t gather;                       // distances come from src; the bounds follow
+  uint32_t stride;                       // uint32 between a source's vertices
+  uint32_t pad;
+  uint64_t dirty16;                      // 16-byte words of the table to clear
+  // src[h][i]: group i's distances to every vertex within hop budget h (h = 0: the distance
+  // table itself); nullptr: unreached
+  const uint32_t* src[HOP_BUDGETS_MAX + 1][KMAX];
 };
-// rows: V distance rows of stride ds (the distance table, or one hop budget's table)
-__global__ void k_gather_dist(uint32_t* rows, uint32_t ds, int k, GroupVecs gv, int64_t V) {
-  for (int64_t v = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; v < V;
-       v += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t d[KMAX];
+__global__ void __launch_bounds__(256) k_admit(Ctx* ctxs, const AdmitQ* aq, int n, DevGraph G) {
+  __shared__ uint32_t s_best[MAXB], s_hop[MAXB];
+  for (int q = threadIdx.x; q < MAXB; q += blockDim.x) s_best[q] = s_hop[q] = COST_INF;
+  __syncthreads();
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < G.V; base += step) {
+    const int64_t v = base + threadIdx.x;
+    const bool live = v < G.V;
+    for (int q = 0; q < n; q++) {
+      const AdmitQ& a = aq[q];
+      Ctx* c = ctxs + a.slot;
+      const int k = c->k, nhb = c->nhb;
+      const uint32_t ds = c->ds;
+      uint32_t best = COST_INF, best_h = COST_INF;
+      if (live) {
+        if (c->rowmap) c->rowmap[v] = ROW_NONE;
+        if ((v & 31) == 0) c->rowbits[v >> 5] = 0u;
+        if (!a.gather || c->phase == PH_SSSP) {
+          if ((v & 3) == 0) c->fm[0][v >> 2] = c->fm[1][v >> 2] = 0u;
+        }
+        const int hs = c->hop && c->sssp_hops && c->D / 2 <= nhb ? c->D / 2 : -1;
+        for (int h = nhb; h >= 0; h--) {
+          uint32_t d[KMAX];
+          uint64_t sum = 0;
 #pragma unroll
-    for (int i = 0; i < KMAX; i++) d[i] = i < k && gv.v[i] ? __ldg(&gv.v[i][v]) : COST_INF;
-    store_drow(rows, ds, (uint64_t)v, make_uint4(d[0], d[1], d[2], d[3]),
-               make_uint4(d[4], d[5], d[6], d[7]));
+          for (int i = 0; i < KMAX; i++) {
+            const uint32_t* src = i < k && a.gather ? a.src[h][i] : nullptr;
+            d[i] = src ? src[v * (int64_t)a.stride] : COST_INF;
+            sum += i < k ? d[i] : 0u;
+          }
+          store_drow(h ? c->dist_h + (uint64_t)(h - 1) * (uint64_t)G.V * ds : c->dist, ds, (uint64_t)v,
+                     make_uint4(d[0], d[1], d[2], d[3]), make_uint4(d[4], d[5], d[6], d[7]));
+          if (h && h == hs) best_h = (uint32_t)min(sum, (uint64_t)COST_INF);
+          if (h == 0 && c->phase == PH_PREP) {
+            best = (uint32_t)min(sum, (uint64_t)COST_INF);
+            if (hs == 0) {  // budget 0: the members themselves
+              bool all = true;
+#pragma unroll
+              for (int i = 0; i < KMAX; i++) all = all && (i >= k || d[i] == 0u);
+              best_h = all ? 0u : COST_INF;
+            }
+#pragma unroll
+            for (int i = 0; i < KMAX; i++)
+              if (i < k && d[i] == 0u) {
+#pragma unroll
+                for (int j = 0; j < KMAX; j++)
+                  if (j < k && d[j] < __ldcg(&c->vv[i * KMAX + j])) atomicMin(&c->vv[i * KMAX + j], d[j]);
+              }
+          }
+        }
+      }
+      best = __reduce_min_sync(0xffffffffu, best);
+      best_h = __reduce_min_sync(0xffffffffu, best_h);
+      if ((threadIdx.x & 31) == 0) {
+        if (best < s_best[q]) atomicMin(&s_best[q], best);
+        if (best_h < s_hop[q]) atomicMin(&s_hop[q], best_h);
+      }
+    }
+  }
+  for (int q = 0; q < n; q++) {
+    uint4* t = (uint4*)ctxs[aq[q].slot].table;
+    const uint64_t m = aq[q].dirty16;
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)step)
+      t[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < n; q += blockDim.x) {
+    Ctx* c = ctxs + aq[q].slot;
+    if (c->phase != PH_PREP) continue;
+    if (s_best[q] < COST_INF) atomicMin(&c->ub, s_best[q]);
+    // ub_cell bounds with strict tests (a state must beat a tree already found), so a
+    // feasible cost that no state holds yet enters it plus one
+    if (s_hop[q] < COST_INF - 1u) atomicMin(&c->ub_cell, s_hop[q] + 1u);
   }
 }
 
 // ---- init: group members -> zero-cost singletons, SSSP sources, dirty rows ----
 // One group per blockIdx.z (KMAX of them): its members' dependent accesses (row map, pool,
 // cell, row list) run beside the other groups' instead of after them.
-__global__ void k_init(Ctx* ctxs, int nctx, DevGraph G, const int64_t* grp_ptr,
-                       const int32_t* members, int split) {
+// aq: the contexts that start (nullptr: all of them).
+__global__ void k_init(Ctx* ctxs, const AdmitQ* aq, int nctx, DevGraph G, const int64_t* grp_ptr,
+                       const int32_t* members) {
   for (int qi = blockIdx.y; qi < nctx; qi += gridDim.y) {
-    Ctx* c = ctxs + qi;
+    Ctx* c = ctxs + (aq ? (int)aq[qi].slot : qi);
     const int i = (int)blockIdx.z;
     if (i < c->k) {
       const int32_t g = c->gid[i];
@@ -1633,11 +1715,12 @@ __device__ __forceinline__ void ctrl_start_dp(Ctx* c) {
 // One block per query context; thread 0 runs the control logic, the whole block
 // builds the tour table when a query leaves its distance phase (in `shared` bytes of
 // dynamic shared memory where they hold it).
-__global__ void __launch_bounds__(512) k_ctrl(Ctx* ctxs, int nctx, int mode, int shared) {
+// aq: the contexts to look at (nullptr: all of them).
+__global__ void __launch_bounds__(512) k_ctrl(Ctx* ctxs, const AdmitQ* aq, int nctx, int mode, int shared) {
   extern __shared__ uint32_t s_tour[];
   const int qi = blockIdx.x;
   if (qi >= nctx) return;
-  Ctx* c = ctxs + qi;
+  Ctx* c = ctxs + (aq ? (int)aq[qi].slot : qi);
   if (mode == CTRL_SSSP && c->phase == PH_PREP && !c->error && c->dist_only) {
     // a group-cache fill: its distances are final, nothing else to build
     if (threadIdx.x == 0) {

@@ -74,20 +74,31 @@ constexpr size_t kTourWords = ((size_t)1 << KMAX) * (TOUR_STRIDE + KMAX + 1);
 constexpr uint32_t kOutCap = 1u << 16;
 constexpr uint32_t kStackCap = 1u << 18;
 
+constexpr size_t kDenseBytes = (size_t)32 << 20;  // tables laid out densely up to here
+constexpr size_t kPoolRoom = (size_t)2 << 30;     // bytes a row pool may take beyond its eighth
+
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Frontier bytes of the distance search: one per vertex (four to a word), padded to
 // whole 16-byte words.
 size_t fm_bytes(int64_t V) { return ((size_t)V + 15) / 16 * 16; }
 
-// Rows of a query's row pool: an eighth of the vertices (at least 64k rows), four times
-// more per capacity retry.  A query writes rows for a few percent of the vertices (its
-// pruning keeps the DP near the optimal trees).  A pool of half the vertices or more
-// becomes the dense layout (one row per vertex, no map): small graphs, last retries.
-uint32_t pool_rows(int64_t V, int boost) {
-  uint64_t r = std::max<uint64_t>(1u << 16, (uint64_t)V / 8);
-  for (int i = 0; i < boost; i++) r *= 4;
-  return r * 2 >= (uint64_t)V ? (uint32_t)V : (uint32_t)r;
+// Rows of a query's row pool: an eighth of the vertices (at least 64k rows), or as many as
+// `room` bytes hold, four times more per capacity retry, at most one per vertex.  Most
+// queries write rows for a few percent of the vertices (their pruning keeps the DP near the
+// optimal trees), but the heaviest k = 7 ones overflow an eighth and then run twice, the
+// second time with a search of their own (10 to 22 of 155 ms of a batch of 32 over 4M
+// vertices, the lost first run not counted: 129 ms without).
+uint32_t pool_rows(int64_t V, size_t rw, size_t room, int boost) {
+  uint64_t r = std::max<uint64_t>(std::max<uint64_t>(1u << 16, (uint64_t)V / 8), room / (rw * 8));
+  for (int i = 0; i < boost; i++) r = std::min<uint64_t>(r * 4, (uint64_t)V);
+  return (uint32_t)std::min<uint64_t>(r, (uint64_t)V);
+}
+// Whether a table of V rows is laid out densely (one row per vertex, no map): where it is
+// small (clearing it costs less than the map's extra reads), and after a capacity retry
+// (a pool of V rows can still run out: a lost race for a row leaves one unused).
+bool dense_rows(int64_t V, size_t rw, uint32_t rows, int boost) {
+  return (int64_t)rows >= V && ((size_t)V * rw * 8 <= kDenseBytes || boost > 0);
 }
 
 // Lay out (or, with base == nullptr, only size) a slot of V vertices: a row pool of
@@ -412,6 +423,9 @@ struct Runner {
   std::vector<Arena> arenas;
   Ctx* d_ctx = nullptr;         // MAXB contexts
   Ctx* h_ctx = nullptr;         // pinned mirror
+  AdmitQ* d_aq = nullptr;       // MAXB: the queries start_admitted() starts
+  AdmitQ* h_aq = nullptr;       // pinned: those admitted since its last call
+  int n_aq = 0;
   uint32_t* d_loop = nullptr;   // graph loop: {iterations left, any query finished}
   uint32_t* loop_init = nullptr;  // pinned: values for d_loop before a launch
   uint32_t* loop_left = nullptr;  // pinned: iterations left after it
@@ -467,6 +481,9 @@ struct Runner {
     held = 0;
     if (d_ctx) cudaFree(d_ctx);
     if (h_ctx) cudaFreeHost(h_ctx);
+    if (d_aq) cudaFree(d_aq);
+    if (h_aq) cudaFreeHost(h_aq);
+    d_aq = h_aq = nullptr;
     if (d_loop) cudaFree(d_loop);
     if (loop_init) cudaFreeHost(loop_init);
     loop_init = loop_left = nullptr;
@@ -478,6 +495,8 @@ struct Runner {
   gst_status init() {
     CK(cudaMalloc(&d_ctx, sizeof(Ctx) * MAXB));
     CK(cudaMallocHost(&h_ctx, sizeof(Ctx) * MAXB));
+    CK(cudaMalloc(&d_aq, sizeof(AdmitQ) * MAXB));
+    CK(cudaMallocHost(&h_aq, sizeof(AdmitQ) * MAXB));
     CK(cudaMalloc(&d_loop, sizeof(uint32_t) * 4));
     CK(cudaMallocHost(&loop_init, sizeof(uint32_t) * 4));
     loop_left = loop_init + 2;
@@ -501,8 +520,21 @@ struct Runner {
     SlotMem tmp;
     const int split = eng->cfg.split_degree;
     const uint32_t cap = list_cap(g->V, g->E, j.rw, split, j.boost);
-    return carve_slot(tmp, nullptr, g->V, j.rw, pool_rows(g->V, j.boost), cap,
+    return carve_slot(tmp, nullptr, g->V, j.rw, job_rows(j), cap,
                       eng->cfg.bucket_delta > 0 ? cap : 0, j.nhb, j.ds);
+  }
+  // a 64th of the budget at most goes to a pool beyond its eighth of the vertices, and
+  // nothing where half the budget would not hold the query then
+  uint32_t job_rows(const Job& j) const {
+    const size_t room = std::min(kPoolRoom, budget / 64);
+    const uint32_t least = pool_rows(g->V, j.rw, 0, j.boost), r = pool_rows(g->V, j.rw, room, j.boost);
+    if (r == least) return r;
+    SlotMem tmp;
+    const uint32_t cap = list_cap(g->V, g->E, j.rw, eng->cfg.split_degree, j.boost);
+    return carve_slot(tmp, nullptr, g->V, j.rw, r, cap, eng->cfg.bucket_delta > 0 ? cap : 0, j.nhb,
+                      j.ds) <= budget / 2
+               ? r
+               : least;
   }
 
   int rw_max() const {
@@ -624,7 +656,7 @@ struct Runner {
     const uint32_t farcap = eng->cfg.bucket_delta > 0 ? cap : 0;
     const size_t need = job_bytes(*j);
     if (need > budget) return GST_OOM_ADMISSION;
-    const size_t need_table = (size_t)pool_rows(g->V, j->boost) * j->rw * 8;
+    const size_t need_table = (size_t)job_rows(*j) * j->rw * 8;
     // the free slot whose memory already fits with the least to spare (a small query
     // does not take a large slot that a large one will want; among equals the lowest,
     // which keeps the contexts the kernels scan few), else the lowest free slot
@@ -647,8 +679,7 @@ struct Runner {
       if (st != GST_OK) return st;
       if (!p) return GST_NOT_READY;
       SlotMem m;
-      carve_slot(m, (unsigned char*)p, g->V, j->rw, pool_rows(g->V, j->boost), cap, farcap, j->nhb,
-                 j->ds);
+      carve_slot(m, (unsigned char*)p, g->V, j->rw, job_rows(*j), cap, farcap, j->nhb, j->ds);
       m.base = p;
       m.bytes = need;
       mem[s] = m;
@@ -699,90 +730,81 @@ struct Runner {
     // then count a cached distance of more edges and come out low; it only sets the
     // search cutoff, which stays non-increasing, so every distance below the final
     // cutoff is still exact and the bounds stay valid.)
-    GroupVecs gv{};
-    const uint32_t* hv[KMAX] = {};
+    AdmitQ& a = h_aq[n_aq];
+    memset(&a, 0, sizeof(a));
+    a.slot = (uint32_t)s;
+    a.stride = 1;
     int n_cached = 0;
     const size_t V = (size_t)g->V;
     if (!hop && !j->cache_dst) {
-      for (int i = 0; i < q->k; i++) n_cached += (gv.v[i] = grp->cache.vec(c.gid[i])) != nullptr;
+      for (int i = 0; i < q->k; i++) n_cached += (a.src[0][i] = grp->cache.vec(c.gid[i])) != nullptr;
     } else if (hop && q->hop_bound > 0 && !j->cache_dst && grp->hop_cache.cap > 0 &&
                grp->hop_cache.D == q->hop_bound) {
-      for (int i = 0; i < q->k; i++) n_cached += (hv[i] = grp->hop_cache.vec(c.gid[i])) != nullptr;
-      for (int i = 0; i < q->k; i++) gv.v[i] = hv[i] ? hv[i] + (size_t)c.nhb * V : nullptr;
+      for (int i = 0; i < q->k; i++) {
+        const uint32_t* hv = grp->hop_cache.vec(c.gid[i]);
+        n_cached += hv != nullptr;
+        for (int h = 0; hv && h <= c.nhb; h++) a.src[h][i] = hv + (size_t)(h ? h - 1 : c.nhb) * V;
+      }
     }
     // a query of the batch-shared search: its distances are in the runner's shared
     // table, exact up to its cutoff; it starts at the bounds pass
     Shared* S = j->ss == 1 ? shared_of(hop ? q->hop_bound : 0) : nullptr;
-    const bool shared = S != nullptr;
-    if (shared) {
-      n_cached = 0;
+    if (S) {
       c.cut_fix = std::max(1u, j->ss_cut);
-      c.phase = PH_PREP;
+      a.stride = S->Gp;
+      for (int h = 0; h <= c.nhb; h++)
+        for (int i = 0; i < q->k; i++) a.src[h][i] = (h ? S->tab[h] : S->dist) + j->ss_cols[i];
+      S->remaining--;
     }
-    const bool cached = n_cached > 0 || shared;
-    if (n_cached == q->k) {
-      c.sssp_full = 1;
-      c.phase = PH_PREP;
-    }
+    a.gather = n_cached > 0 || S;
+    if (S || n_cached == q->k) c.phase = PH_PREP;
+    if (!S && n_cached == q->k) c.sssp_full = 1;
     c.sssp_mask = c.sssp_hops ? 2u : (c.bucket_end == 0xFFFFFFFFu ? 1u : 0u);
-    cudaStream_t st = eng->stream;
     // the pool takes every row the slot's table holds; only the rows the slot's last
     // query wrote need clearing
     c.pool_cap = (uint32_t)std::min<uint64_t>((uint64_t)g->V, m.table_bytes / ((size_t)c.RW * 8));
     c.pool_n = 0;
-    if (c.pool_cap >= (uint32_t)g->V) c.rowmap = nullptr;  // a row for every vertex: dense
-    if (m.table_dirty) CK(cudaMemsetAsync(m.table, 0xFF, m.table_dirty, st));
+    if (dense_rows(g->V, (size_t)c.RW, c.pool_cap, j->boost)) c.rowmap = nullptr;
+    a.dirty16 = (m.table_dirty + 15) / 16;
     m.table_dirty = 0;
-    if (c.rowmap) CK(cudaMemsetAsync(m.rowmap, 0xFF, (size_t)g->V * 4, st));
-    CK(cudaMemsetAsync(m.rowbits, 0, ((size_t)g->V + 31) / 32 * 4, st));
-    if (c.use_lb && !cached) CK(cudaMemsetAsync(m.dist, 0xFF, (size_t)g->V * c.ds * 4, st));
-    CK(cudaMemsetAsync(m.fm[0], 0, fm_bytes(g->V), st));
-    CK(cudaMemsetAsync(m.fm[1], 0, fm_bytes(g->V), st));
-    if (c.nhb && !cached)
-      CK(cudaMemsetAsync(m.dist_h, 0xFF, (size_t)c.nhb * (size_t)g->V * c.ds * 4, st));
-    CK(cudaMemcpyAsync(d_ctx + s, &c, sizeof(Ctx), cudaMemcpyHostToDevice, st));
-    cs.h2d += sizeof(Ctx) + sizeof(int32_t) * q->k;
-    const DevGraph G = dev_graph(g);
-    if (shared) {
-      // the distance table, and for a hop-bounded query its budgets 1..nhb
-      const uint16_t* sc = j->ss_cols;
-      const ushort4 c0 = make_ushort4(sc[0], sc[1], sc[2], sc[3]);
-      const ushort4 c1 = make_ushort4(sc[4], sc[5], sc[6], sc[7]);
-      k_bs_gather<<<eng->sssp_blocks, 256, 0, st>>>(m.dist, c.ds, q->k, S->dist, S->Gp, c0, c1, g->V);
-      cs.launches += 1;
-      for (int h = 1; h <= c.nhb; h++) {
-        k_bs_gather<<<eng->sssp_blocks, 256, 0, st>>>(m.dist_h + (size_t)(h - 1) * V * c.ds, c.ds,
-                                                      q->k, S->tab[h], S->Gp, c0, c1, g->V);
-        cs.launches += 1;
-      }
-      S->remaining--;
-    } else if (cached) {
-      k_gather_dist<<<eng->sssp_blocks, 256, 0, st>>>(m.dist, c.ds, q->k, gv, g->V);
-      cs.launches += 1;
-      if (hop)
-        for (int h = 1; h <= c.nhb; h++) {
-          GroupVecs gh{};
-          for (int i = 0; i < q->k; i++) gh.v[i] = hv[i] ? hv[i] + (size_t)(h - 1) * V : nullptr;
-          k_gather_dist<<<eng->sssp_blocks, 256, 0, st>>>(
-              m.dist_h + (size_t)(h - 1) * V * c.ds, c.ds, q->k, gh, g->V);
-          cs.launches += 1;
-        }
-    }
-    k_init<<<dim3(8, 1, KMAX), 256, 0, st>>>(d_ctx + s, 1, G, grp->d_ptr, grp->d_mem,
-                                       eng->cfg.split_degree);
-    if (n_cached == q->k || shared) {
-      // the bounds pass over the distance rows (star bound, group distances), which
-      // the control step after it turns into the tour table
-      k_sssp<<<eng->sssp_blocks, 256, 0, st>>>(d_ctx + s, 1, G, eng->cfg.split_degree);
-      cs.launches += 1;
-    }
-    const int tour_bytes = c.W * TOUR_STRIDE * 4;
-    k_ctrl<<<1, 512, tour_bytes, st>>>(d_ctx + s, 1, CTRL_SSSP, tour_bytes);
-    cs.launches += 2;
+    n_aq++;
     owner[s] = j;
     idle_written[s] = 0;
     nctx = std::max(nctx, s + 1);
     active++;
+    return GST_OK;
+  }
+
+  // Upload and start the queries admitted since the last call, all in the same launches:
+  // their buffers and distances (k_admit), their seeds, and their first control step, which
+  // builds the tour tables of those whose distances are final.
+  gst_status start_admitted() {
+    if (n_aq == 0) return GST_OK;
+    cudaStream_t st = eng->stream;
+    const DevGraph G = dev_graph(g);
+    const int n = n_aq;
+    n_aq = 0;
+    int kmax = 1;
+    for (int i = 0; i < n; i++) {
+      const uint32_t s = h_aq[i].slot;
+      kmax = std::max(kmax, h_ctx[s].k);
+      int run = 1;  // neighbouring slots go in one copy
+      while (i + run < n && h_aq[i + run].slot == s + (uint32_t)run) {
+        kmax = std::max(kmax, h_ctx[s + run].k);
+        run++;
+      }
+      CK(cudaMemcpyAsync(d_ctx + s, h_ctx + s, sizeof(Ctx) * run, cudaMemcpyHostToDevice, st));
+      i += run - 1;
+    }
+    CK(cudaMemcpyAsync(d_aq, h_aq, sizeof(AdmitQ) * n, cudaMemcpyHostToDevice, st));
+    cs.h2d += (int64_t)(sizeof(Ctx) + sizeof(AdmitQ)) * n;
+    const int blocks = (int)std::min<int64_t>(eng->sms * 8, (g->V + 255) / 256);
+    k_admit<<<blocks, 256, 0, st>>>(d_ctx, d_aq, n, G);
+    k_init<<<dim3(8, n, KMAX), 256, 0, st>>>(d_ctx, d_aq, n, G, grp->d_ptr, grp->d_mem);
+    const int tour_bytes = (1 << kmax) * TOUR_STRIDE * 4;
+    k_ctrl<<<n, 512, tour_bytes, st>>>(d_ctx, d_aq, n, CTRL_SSSP, tour_bytes);
+    cs.launches += 3;
+    CK(cudaGetLastError());
     return GST_OK;
   }
 
@@ -815,6 +837,12 @@ struct Runner {
   // cutoff; without memory for the tables, or when the search reports an error, the jobs
   // keep their own searches.
   gst_status shared_search(const std::vector<Job*>& jobs, const std::vector<int32_t>& cols, int D) {
+    gst_status s = GST_OK;
+    if (n_aq) {  // nothing admitted reads memory that is taken below
+      s = start_admitted();
+      if (s != GST_OK) return s;
+      CK(cudaStreamSynchronize(eng->stream));  // h_aq is free again
+    }
     const int64_t V = g->V;
     const uint32_t ncols = (uint32_t)cols.size();
     const uint32_t Gp = (ncols + 7u) / 8u * 8u, Wm = (Gp + 31u) / 32u;
@@ -841,7 +869,7 @@ struct Runner {
     const size_t o_items = take((size_t)item_cap * 8);
     const size_t o_cols = take((size_t)BS_COLS * 4);
     void* p = nullptr;
-    gst_status s = slot_memory(off, &p);
+    s = slot_memory(off, &p);
     if (s != GST_OK) return s;
     if (!p) return GST_OK;  // no room: the queries search on their own
     unsigned char* base = (unsigned char*)p;
@@ -1004,7 +1032,7 @@ struct Runner {
       const int pe = prof ? prof_begin(PROF_SSSP) : -1;
       k_sssp<<<eng->sssp_blocks, 256, 0, st>>>(d_ctx, nctx, G, split);
       prof_end(pe);
-      k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nctx, CTRL_SSSP, 0);
+      k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nullptr, nctx, CTRL_SSSP, 0);
     }
     const size_t per_warp = rows_smem_per_warp(rwm);
     // k_rows: at most 256 threads, as many warps as the widest row lets fit
@@ -1013,11 +1041,11 @@ struct Runner {
     k_rows<<<rows_blocks(eng, warps * 32, per_warp * warps), warps * 32, per_warp * warps, st>>>(
         d_ctx, nctx, G, split, rwm);
     prof_end(pe);
-    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nctx, CTRL_DP_ROWS, 0);
+    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nullptr, nctx, CTRL_DP_ROWS, 0);
     pe = prof ? prof_begin(PROF_GROW) : -1;
     k_grow<<<eng->grow_blocks, 256, 0, st>>>(d_ctx, nctx, G, split);
     prof_end(pe);
-    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nctx, CTRL_DP_GROW, 0);
+    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nullptr, nctx, CTRL_DP_GROW, 0);
   }
 
   // The level loop as a CUDA graph: a WHILE node whose body is one level plus a
@@ -1070,7 +1098,8 @@ struct Runner {
   // max_levels > 0, at most about that many levels), then read the contexts.
   gst_status run(int max_levels) {
     {
-      gst_status s = write_idle();
+      gst_status s = start_admitted();
+      if (s == GST_OK) s = write_idle();
       if (s != GST_OK) return s;
     }
     const int rwm = rw_max();
@@ -1154,6 +1183,9 @@ struct Runner {
                              !cap_is_worst(g->V, g->E, j->rw, eng->cfg.split_degree, c.qcap);
       const bool pool_full = (c.error & ERR_POOL) && c.rowmap != nullptr;
       if (list_full || pool_full) {
+        if (eng->cfg.verbose)
+          fprintf(stderr, "[gst retry] k %d D %d: error bits 0x%x, pool %u of %u rows\n", c.k,
+                  j->q.hop_bound, c.error, c.pool_n, c.pool_cap);
         j->boost++;
         j->ss = 0;  // a retry searches on its own
         retry.push_back(j);
@@ -2617,19 +2649,19 @@ gst_status noalloc_solve(int device, cudaStream_t st, int64_t V, int64_t E, cons
   NCK(cudaMemcpyAsync(d_ctx, &c, sizeof(Ctx), cudaMemcpyHostToDevice, st));
   // the caller's edges are sorted by neighbour only: no light-edge index
   DevGraph G{V, E, d_beg, (const int2*)d_edges, (const int2*)d_edges, nullptr, 0u};
-  k_init<<<dim3(8, 1, KMAX), 256, 0, st>>>(d_ctx, 1, G, d_grp_ptr, d_members, split);
-  k_ctrl<<<1, 32, 0, st>>>(d_ctx, 1, CTRL_SSSP, 0);
+  k_init<<<dim3(8, 1, KMAX), 256, 0, st>>>(d_ctx, nullptr, 1, G, d_grp_ptr, d_members);
+  k_ctrl<<<1, 32, 0, st>>>(d_ctx, nullptr, 1, CTRL_SSSP, 0);
   const size_t smem = rows_smem_per_warp((int)RW) * (size_t)warps;
   int64_t launches = 2;
   Ctx h;
   for (;;) {
     for (int i = 0; i < 6; i++) {
       k_sssp<<<nd->sssp_blocks, 256, 0, st>>>(d_ctx, 1, G, split);
-      k_ctrl<<<1, 128, 0, st>>>(d_ctx, 1, CTRL_SSSP, 0);
+      k_ctrl<<<1, 128, 0, st>>>(d_ctx, nullptr, 1, CTRL_SSSP, 0);
       k_rows<<<nd->sms * 4, warps * 32, smem, st>>>(d_ctx, 1, G, split, (int)RW);
-      k_ctrl<<<1, 128, 0, st>>>(d_ctx, 1, CTRL_DP_ROWS, 0);
+      k_ctrl<<<1, 128, 0, st>>>(d_ctx, nullptr, 1, CTRL_DP_ROWS, 0);
       k_grow<<<nd->grow_blocks, 256, 0, st>>>(d_ctx, 1, G, split);
-      k_ctrl<<<1, 128, 0, st>>>(d_ctx, 1, CTRL_DP_GROW, 0);
+      k_ctrl<<<1, 128, 0, st>>>(d_ctx, nullptr, 1, CTRL_DP_GROW, 0);
       launches += 6;
     }
     NCK(cudaGetLastError());
