@@ -90,21 +90,6 @@ struct BsCtx {
 };
 constexpr uint32_t BS_ERR_ITEMS = 1, BS_ERR_STEPS = 2;
 
-// True in the last block of the grid to get here, which then sees the other blocks'
-// writes; no block waits.  All threads of every block call it once per launch.
-__device__ __forceinline__ bool last_block(uint32_t* arrived) {
-  __shared__ bool s_last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s_last = atomicAdd(arrived, 1u) == gridDim.x - 1u;
-    if (s_last) *arrived = 0u;
-  }
-  __syncthreads();
-  if (s_last) __threadfence();
-  return s_last;
-}
-
 // First and one-past-last edge of v's weight-sorted list in the current class.
 __device__ __forceinline__ void class_range(const BsCtx* b, uint32_t cls, uint32_t v, int64_t deg,
                                             int64_t* lo, int64_t* hi) {

@@ -99,7 +99,6 @@ enum Phase : uint32_t { PH_SSSP = 0, PH_PREP = 1, PH_DP = 2, PH_DONE = 3, PH_ERR
 enum ErrBits : uint32_t { ERR_QCAP = 1, ERR_FARCAP = 2, ERR_ROWCAP = 4, ERR_TIMEOUT = 8,
                           ERR_EXTRACT = 16, ERR_BOUNDS = 32, ERR_POOL = 64 };
 constexpr uint32_t ROW_NONE = 0xFFFFFFFFu;
-enum CtrlMode : int { CTRL_SSSP = 0, CTRL_DP_ROWS = 1, CTRL_DP_GROW = 2 };
 
 // Light-edge index: per vertex, the number of edges of weight <= widx_threshold(t) << wsh
 // for t < WIDX, thresholds 1, 2, 3, 4, 6, 8, 12, ..., 192, 256 (each step x1.5 or
@@ -112,6 +111,7 @@ enum CtrlMode : int { CTRL_SSSP = 0, CTRL_DP_ROWS = 1, CTRL_DP_GROW = 2 };
 // (grow 4.6 to 3.1 ms, the call 15.2 to 13.6 ms).
 constexpr int WIDX = 16;
 constexpr uint32_t CHUNK = 0x80000000u;  // item flag (in pd): one `split`-edge chunk only
+constexpr uint32_t GROW_TAKE = 16;       // grow items a warp takes at a time, at most
 constexpr int RELAX_U = 4;               // edges per lane per round of the grow relax loop
 // Hop-limited distance items carry their path's edge count in bits 8..15 of the
 // group word (group index in bits 0..7).
@@ -348,6 +348,21 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x) {
     if (lane >= o) x += y;
   }
   return x;
+}
+
+// True in the last block of the grid to get here, which then sees the other blocks'
+// writes; no block waits.  All threads of every block call it once per launch.
+__device__ __forceinline__ bool last_block(uint32_t* arrived) {
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_last = atomicAdd(arrived, 1u) == gridDim.x - 1u;
+    if (s_last) *arrived = 0u;
+  }
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last;
 }
 
 // ---- worklists -----------------------------------------------------------------
@@ -1056,16 +1071,94 @@ __global__ void __launch_bounds__(256, 4) k_sssp(Ctx* ctxs, int nctx, DevGraph G
   }
 }
 
+// ---- control: one thread per query -------------------------------------------------
+// Words of a level loop, in device memory.
+struct LoopCtl {
+  uint32_t left;        // graph loop: iterations left (host-set before the launch)
+  uint32_t arrived[2];  // blocks of the current rows / grow launch that are done
+  uint32_t next;        // grow items taken from the counter in the current launch
+};
+__device__ __forceinline__ void ctrl_take_far(Ctx* c) {
+  // advance the cost bucket and take the far list as the next input
+  const uint32_t fm = c->far_min;
+  c->bucket_end = (c->delta == 0) ? 0xFFFFFFFFu
+                                  : (uint32_t)min((uint64_t)fm + c->delta, (uint64_t)0xFFFFFFFFu);
+  c->in_ptr = c->far[c->f];
+  c->in_n = min(c->n_far[c->f], c->farcap);
+  c->in_kind = 1;
+  c->in_idx = c->f;
+  c->f ^= 1u;
+  c->n_far[c->f] = 0;
+  c->far_min = 0xFFFFFFFFu;
+}
+
+// After the rows kernel: it appended the grow items of the states it settled to q[no]
+// (after the continuations the last grow step appended there).
+__device__ __forceinline__ void ctrl_rows(Ctx* c) {
+  if (c->phase >= PH_DONE) return;
+  if (c->error) {
+    c->phase = PH_ERROR;
+    c->in_n = 0;
+    return;
+  }
+  if (c->phase != PH_DP) return;
+  c->n_rows = 0;  // consumed by the rows kernel
+  const uint32_t s = c->no;
+  c->st_qmax = max(c->st_qmax, max(c->n_q[s], c->n_far[c->f]));
+  if (c->n_q[s] > 0) {
+    c->in_ptr = c->q[s];
+    c->in_n = min(c->n_q[s], c->qcap);
+    c->in_kind = 0;
+    c->in_idx = s;
+    c->no = s ^ 1u;
+  } else if (c->n_far[c->f] > 0) {
+    ctrl_take_far(c);
+  } else {
+    c->phase = PH_DONE;
+    c->in_n = 0;
+  }
+}
+// After the grow kernel: its input list is empty again; the level budget.
+__device__ __forceinline__ void ctrl_grow(Ctx* c) {
+  if (c->phase >= PH_DONE) return;
+  if (c->error) {
+    c->phase = PH_ERROR;
+    c->in_n = 0;
+    return;
+  }
+  if (c->phase != PH_DP) return;
+  if (++c->levels > c->max_levels) {
+    c->error |= ERR_TIMEOUT;
+    c->phase = PH_ERROR;
+    c->in_n = 0;
+    return;
+  }
+  if (c->in_kind == 0) c->n_q[c->in_idx] = 0;
+  else c->n_far[c->in_idx] = 0;
+  c->in_n = 0;
+}
+
 // ---- DP grow step ----------------------------------------------------------------
-__global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G, int split) {
+// A warp takes up to GROW_TAKE items at a time, fewer where that spreads a level over all
+// warps: a head item may stand for `split` edges, and 32 of them in one warp were a serial
+// chain of 0.3-0.5 ms in levels of a few thousand items, 13 % of the warps active.  The
+// first take of a warp is its own share, the further ones come from a counter.  Three
+// hop-bounded queries over 1M vertices: grow 4.7 to 1.4 ms, three queries k = 5/7 over
+// 141k: 3.0 to 1.5 ms.  With 8 items at most the 141k batch takes 5.6 ms instead of 4.9,
+// with 32 the 1M batch 4.0 instead of 3.4.
+// The last block runs the control step of every query; in the graph loop (in_loop) it
+// also decides whether the loop goes on: no resident query has finished,
+// some query is resident, iterations are left.
+__global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G, int split, LoopCtl* lc,
+                                              cudaGraphConditionalHandle loop, int in_loop) {
   __shared__ uint32_t s_pref[MAXB + 1];
   load_prefix(ctxs, nctx, s_pref, PH_DP);
   const uint32_t total = s_pref[nctx];
   const int lane = threadIdx.x & 31;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  for (uint32_t base = wid * 32; base < total; base += warps * 32) {
-    const uint32_t it = base + lane;
+  const uint32_t take = max(1u, min(GROW_TAKE, (total + warps - 1u) / warps));
+  for (uint32_t base = ((threadIdx.x >> 5) * gridDim.x + blockIdx.x) * take; base < total;) {
+    const uint32_t it = (uint32_t)lane < take ? base + lane : total;
     uint32_t v = 0, pd = 0, cost = 0, bound = 0, e_off = 0, wmax = 0;
     bool chunk = false;
     int qi = 0;
@@ -1220,6 +1313,25 @@ __global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G
         warp_mark_row(ctxs, x_qi[x], dirty, u);
       }
     }
+    if (lane == 0) base = warps * take + atomicAdd(&lc->next, take);
+    base = __shfl_sync(0xffffffffu, base, 0);
+  }
+  if (!last_block(&lc->arrived[1])) return;
+  const int i = threadIdx.x;  // blockDim.x >= MAXB
+  bool fin = false, act = false;
+  if (i < nctx) {
+    ctrl_grow(ctxs + i);
+    act = !ctxs[i].idle;
+    fin = act && ctxs[i].phase >= PH_DONE;
+  }
+  const int any_fin = __syncthreads_or(fin), any_act = __syncthreads_or(act);
+  if (i == 0) {
+    lc->next = 0u;
+    if (in_loop) {
+      const uint32_t left = lc->left > 0 ? lc->left - 1u : 0u;
+      lc->left = left;
+      cudaGraphSetConditional(loop, (!any_fin && any_act && left > 0) ? 1u : 0u);
+    }
   }
 }
 
@@ -1233,8 +1345,9 @@ __host__ __device__ __forceinline__ size_t rows_smem_per_warp(int rw_max) {
 }
 
 // Dynamic shared memory per warp: RWmax cells + RWmax/32 pending words + RWmax list.
-__global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G, int split,
-                                              int rw_max) {
+// The last block runs the control step of every query.
+__global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G, int rw_max,
+                                              LoopCtl* lc) {
   __shared__ uint32_t s_pref[MAXB + 1];
   extern __shared__ __align__(16) unsigned char s_dyn[];
   load_prefix(ctxs, nctx, s_pref, -1);
@@ -1616,21 +1729,8 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
     atomicAdd(&ctxs[st_q].st_merge, (unsigned long long)st_merges);
     atomicAdd(&ctxs[st_q].st_rows, (unsigned long long)st_rows);
   }
-}
-
-// ---- control: one thread per query -------------------------------------------------
-__device__ __forceinline__ void ctrl_take_far(Ctx* c) {
-  // advance the cost bucket and take the far list as the next input
-  const uint32_t fm = c->far_min;
-  c->bucket_end = (c->delta == 0) ? 0xFFFFFFFFu
-                                  : (uint32_t)min((uint64_t)fm + c->delta, (uint64_t)0xFFFFFFFFu);
-  c->in_ptr = c->far[c->f];
-  c->in_n = min(c->n_far[c->f], c->farcap);
-  c->in_kind = 1;
-  c->in_idx = c->f;
-  c->f ^= 1u;
-  c->n_far[c->f] = 0;
-  c->far_min = 0xFFFFFFFFu;
+  if (!last_block(&lc->arrived[0])) return;
+  for (int i = threadIdx.x; i < nctx; i += blockDim.x) ctrl_rows(ctxs + i);
 }
 
 // Tour table of one query (all threads of the block): P[X][i][j] = cheapest
@@ -1712,16 +1812,16 @@ __device__ __forceinline__ void ctrl_start_dp(Ctx* c) {
   c->bucket_end = c->delta ? c->delta : 0xFFFFFFFFu;
 }
 
-// One block per query context; thread 0 runs the control logic, the whole block
-// builds the tour table when a query leaves its distance phase (in `shared` bytes of
+// Control of the distance phase: one block per query context; thread 0 runs the control
+// logic, the whole block builds the tour table when a query leaves its distance phase (in `shared` bytes of
 // dynamic shared memory where they hold it).
 // aq: the contexts to look at (nullptr: all of them).
-__global__ void __launch_bounds__(512) k_ctrl(Ctx* ctxs, const AdmitQ* aq, int nctx, int mode, int shared) {
+__global__ void __launch_bounds__(512) k_ctrl(Ctx* ctxs, const AdmitQ* aq, int nctx, int shared) {
   extern __shared__ uint32_t s_tour[];
   const int qi = blockIdx.x;
   if (qi >= nctx) return;
   Ctx* c = ctxs + (aq ? (int)aq[qi].slot : qi);
-  if (mode == CTRL_SSSP && c->phase == PH_PREP && !c->error && c->dist_only) {
+  if (c->phase == PH_PREP && !c->error && c->dist_only) {
     // a group-cache fill: its distances are final, nothing else to build
     if (threadIdx.x == 0) {
       c->phase = PH_DONE;
@@ -1729,7 +1829,7 @@ __global__ void __launch_bounds__(512) k_ctrl(Ctx* ctxs, const AdmitQ* aq, int n
     }
     return;
   }
-  if (mode == CTRL_SSSP && c->phase == PH_PREP && !c->error) {
+  if (c->phase == PH_PREP && !c->error) {
     // The distances are final up to the cutoff ub: every stored distance <= ub is
     // exact, and any other is only known to be > ub.  The group distances feed a
     // lower bound, so they are clamped to ub + 1, a value never above the truth.
@@ -1752,89 +1852,32 @@ __global__ void __launch_bounds__(512) k_ctrl(Ctx* ctxs, const AdmitQ* aq, int n
     c->in_n = 0;
     return;
   }
-  if (mode == CTRL_SSSP) {
-    if (c->phase != PH_SSSP) return;
-    if (++c->levels > c->max_levels) {
-      c->error |= ERR_TIMEOUT;
-      c->phase = PH_ERROR;
-      c->in_n = 0;
-      return;
-    }
-    // the finished step read in_ptr and pushed near items into q[no]
-    if (c->in_kind == 0) c->n_q[c->in_idx] = 0;
-    else c->n_far[c->in_idx] = 0;
-    const uint32_t s = c->no;
-    c->st_qmax = max(c->st_qmax, max(c->n_q[s], c->n_far[c->f]));
-    if (c->n_q[s] > 0) {
-      c->in_ptr = c->q[s];
-      c->in_n = min(c->n_q[s], c->qcap);
-      c->in_kind = 0;
-      c->in_idx = s;
-      c->no = s ^ 1u;
-    } else if (c->n_far[c->f] > 0) {
-      ctrl_take_far(c);
-      c->no = s;
-    } else {
-      // distances final: the next k_sssp launch builds the bounds (PH_PREP), the
-      // control step after it the tour table, then the DP starts
-      c->phase = PH_PREP;
-      c->in_n = 0;
-    }
-  } else if (mode == CTRL_DP_ROWS) {
-    // the rows kernel appended the grow items of the states it settled to q[no]
-    // (after the continuations the last grow step appended there)
-    if (c->phase != PH_DP) return;
-    c->n_rows = 0;  // consumed by the rows kernel
-    const uint32_t s = c->no;
-    c->st_qmax = max(c->st_qmax, max(c->n_q[s], c->n_far[c->f]));
-    if (c->n_q[s] > 0) {
-      c->in_ptr = c->q[s];
-      c->in_n = min(c->n_q[s], c->qcap);
-      c->in_kind = 0;
-      c->in_idx = s;
-      c->no = s ^ 1u;
-    } else if (c->n_far[c->f] > 0) {
-      ctrl_take_far(c);
-    } else {
-      c->phase = PH_DONE;
-      c->in_n = 0;
-    }
-  } else {  // CTRL_DP_GROW
-    if (c->phase != PH_DP) return;
-    if (++c->levels > c->max_levels) {
-      c->error |= ERR_TIMEOUT;
-      c->phase = PH_ERROR;
-      c->in_n = 0;
-      return;
-    }
-    if (c->in_kind == 0) c->n_q[c->in_idx] = 0;
-    else c->n_far[c->in_idx] = 0;
+  if (c->phase != PH_SSSP) return;
+  if (++c->levels > c->max_levels) {
+    c->error |= ERR_TIMEOUT;
+    c->phase = PH_ERROR;
     c->in_n = 0;
+    return;
   }
-}
-
-// ---- device-side loop control of the level graph -----------------------------------
-// Last node of the level body of the CUDA graph's WHILE loop: go on while no
-// resident query has finished, some query is resident and iterations are left.
-// loop[0] = iterations left (host-set before the launch), loop[1] = a query finished.
-__global__ void k_loop_cond(const Ctx* ctxs, int nctx, uint32_t* loop,
-                            cudaGraphConditionalHandle h) {
-  const int i = threadIdx.x;  // blockDim.x >= MAXB
-  bool fin = false, act = false;
-  if (i < nctx) {
-    const Ctx* c = ctxs + i;
-    if (!c->idle) {
-      act = true;
-      fin = c->phase >= PH_DONE;
-    }
-  }
-  const int any_fin = __syncthreads_or(fin);
-  const int any_act = __syncthreads_or(act);
-  if (i == 0) {
-    const uint32_t left = loop[0] > 0 ? loop[0] - 1u : 0u;
-    loop[0] = left;
-    loop[1] = any_fin ? 1u : 0u;
-    cudaGraphSetConditional(h, (!any_fin && any_act && left > 0) ? 1u : 0u);
+  // the finished step read in_ptr and pushed near items into q[no]
+  if (c->in_kind == 0) c->n_q[c->in_idx] = 0;
+  else c->n_far[c->in_idx] = 0;
+  const uint32_t s = c->no;
+  c->st_qmax = max(c->st_qmax, max(c->n_q[s], c->n_far[c->f]));
+  if (c->n_q[s] > 0) {
+    c->in_ptr = c->q[s];
+    c->in_n = min(c->n_q[s], c->qcap);
+    c->in_kind = 0;
+    c->in_idx = s;
+    c->no = s ^ 1u;
+  } else if (c->n_far[c->f] > 0) {
+    ctrl_take_far(c);
+    c->no = s;
+  } else {
+    // distances final: the next k_sssp launch builds the bounds (PH_PREP), the
+    // control step after it the tour table, then the DP starts
+    c->phase = PH_PREP;
+    c->in_n = 0;
   }
 }
 

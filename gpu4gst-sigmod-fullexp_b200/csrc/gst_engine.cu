@@ -426,19 +426,21 @@ struct Runner {
   AdmitQ* d_aq = nullptr;       // MAXB: the queries start_admitted() starts
   AdmitQ* h_aq = nullptr;       // pinned: those admitted since its last call
   int n_aq = 0;
-  uint32_t* d_loop = nullptr;   // graph loop: {iterations left, any query finished}
+  LoopCtl* d_loop = nullptr;    // counters of the level loop
   uint32_t* loop_init = nullptr;  // pinned: values for d_loop before a launch
   uint32_t* loop_left = nullptr;  // pinned: iterations left after it
   std::vector<SlotMem> mem;
   std::vector<Job*> owner;      // slot -> job (nullptr = free)
   std::vector<uint8_t> idle_written;
+  std::vector<uint8_t> searching;  // the slot's query is in its own distance search
   int nctx = 0;                 // slots the kernels scan (high-water mark)
   int active = 0;
   CallStats cs;
-  // CUDA graphs of the level loop, by (nctx, rw_max)
+  // CUDA graphs of the level loop, by (nctx, rw_max, sssp)
   struct LoopGraph {
     int nctx;
     int rw_max;
+    bool sssp;  // the body holds the distance search of single queries
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
   };
@@ -497,12 +499,14 @@ struct Runner {
     CK(cudaMallocHost(&h_ctx, sizeof(Ctx) * MAXB));
     CK(cudaMalloc(&d_aq, sizeof(AdmitQ) * MAXB));
     CK(cudaMallocHost(&h_aq, sizeof(AdmitQ) * MAXB));
-    CK(cudaMalloc(&d_loop, sizeof(uint32_t) * 4));
+    CK(cudaMalloc(&d_loop, sizeof(LoopCtl)));
+    CK(cudaMemset(d_loop, 0, sizeof(LoopCtl)));
     CK(cudaMallocHost(&loop_init, sizeof(uint32_t) * 4));
     loop_left = loop_init + 2;
     mem.assign(max_slots, SlotMem());
     owner.assign(max_slots, nullptr);
     idle_written.assign(max_slots, 0);
+    searching.assign(max_slots, 0);
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
     // memory the engine's pool keeps but no allocation uses (arenas released by another
@@ -769,6 +773,7 @@ struct Runner {
     m.table_dirty = 0;
     n_aq++;
     owner[s] = j;
+    searching[s] = c.phase == PH_SSSP;
     idle_written[s] = 0;
     nctx = std::max(nctx, s + 1);
     active++;
@@ -802,7 +807,7 @@ struct Runner {
     k_admit<<<blocks, 256, 0, st>>>(d_ctx, d_aq, n, G);
     k_init<<<dim3(8, n, KMAX), 256, 0, st>>>(d_ctx, d_aq, n, G, grp->d_ptr, grp->d_mem);
     const int tour_bytes = (1 << kmax) * TOUR_STRIDE * 4;
-    k_ctrl<<<n, 512, tour_bytes, st>>>(d_ctx, d_aq, n, CTRL_SSSP, tour_bytes);
+    k_ctrl<<<n, 512, tour_bytes, st>>>(d_ctx, d_aq, n, tour_bytes);
     cs.launches += 3;
     CK(cudaGetLastError());
     return GST_OK;
@@ -1023,8 +1028,10 @@ struct Runner {
     if (i >= 0) cudaEventRecord(eng->prof_events[2 * i + 1], eng->stream);
   }
 
-  // One level of every resident query: sssp, ctrl, rows, ctrl, grow, ctrl.
-  void launch_level(cudaStream_t st, int rwm, bool sssp, bool prof) {
+  // One level of every resident query: rows, grow, each with its control step (and before
+  // them, while some query searches its own distances, sssp and ctrl).  `loop`: the graph
+  // loop's handle (nullptr outside of it).
+  void launch_level(cudaStream_t st, int rwm, bool sssp, bool prof, const cudaGraphConditionalHandle* loop) {
     const DevGraph G = dev_graph(g);
     const int split = eng->cfg.split_degree;
     const int tpb = eng->cfg.threads_per_block;
@@ -1032,33 +1039,33 @@ struct Runner {
       const int pe = prof ? prof_begin(PROF_SSSP) : -1;
       k_sssp<<<eng->sssp_blocks, 256, 0, st>>>(d_ctx, nctx, G, split);
       prof_end(pe);
-      k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nullptr, nctx, CTRL_SSSP, 0);
+      k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nullptr, nctx, 0);
     }
     const size_t per_warp = rows_smem_per_warp(rwm);
     // k_rows: at most 256 threads, as many warps as the widest row lets fit
     const int warps = rows_warps(eng->rows_smem, tpb, rwm);
     int pe = prof ? prof_begin(PROF_ROWS) : -1;
     k_rows<<<rows_blocks(eng, warps * 32, per_warp * warps), warps * 32, per_warp * warps, st>>>(
-        d_ctx, nctx, G, split, rwm);
+        d_ctx, nctx, G, rwm, d_loop);
     prof_end(pe);
-    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nullptr, nctx, CTRL_DP_ROWS, 0);
     pe = prof ? prof_begin(PROF_GROW) : -1;
-    k_grow<<<eng->grow_blocks, 256, 0, st>>>(d_ctx, nctx, G, split);
+    k_grow<<<eng->grow_blocks, 256, 0, st>>>(d_ctx, nctx, G, split, d_loop,
+                                             loop ? *loop : cudaGraphConditionalHandle{}, loop != nullptr);
     prof_end(pe);
-    k_ctrl<<<nctx, 128, 0, st>>>(d_ctx, nullptr, nctx, CTRL_DP_GROW, 0);
   }
 
-  // The level loop as a CUDA graph: a WHILE node whose body is one level plus a
-  // kernel that decides whether to go on (no query finished, iterations left).
-  gst_status loop_graph(int rwm, cudaGraphExec_t* out) {
+  // The level loop as a CUDA graph: a WHILE node whose body is one level, whose grow kernel
+  // decides whether to go on (no query finished, iterations left).
+  gst_status loop_graph(int rwm, bool sssp, cudaGraphExec_t* out) {
     for (auto& lg : graphs)
-      if (lg.nctx == nctx && lg.rw_max == rwm) {
+      if (lg.nctx == nctx && lg.rw_max == rwm && lg.sssp == sssp) {
         *out = lg.exec;
         return GST_OK;
       }
     LoopGraph lg;
     lg.nctx = nctx;
     lg.rw_max = rwm;
+    lg.sssp = sssp;
     CK(cudaGraphCreate(&lg.graph, 0));
     cudaGraphConditionalHandle handle;
     CK(cudaGraphConditionalHandleCreate(&handle, lg.graph, 1, cudaGraphCondAssignDefault));
@@ -1079,8 +1086,7 @@ struct Runner {
     CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
     CK(cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0,
                                      cudaStreamCaptureModeThreadLocal));
-    launch_level(cap, rwm, true, false);
-    k_loop_cond<<<1, 64, 0, cap>>>(d_ctx, nctx, d_loop, handle);
+    launch_level(cap, rwm, sssp, false, &handle);
     cudaGraph_t captured = nullptr;
     cudaError_t ce = cudaStreamEndCapture(cap, &captured);
     cudaStreamDestroy(cap);
@@ -1103,28 +1109,28 @@ struct Runner {
       if (s != GST_OK) return s;
     }
     const int rwm = rw_max();
-    bool any_sssp = true;
+    bool any_sssp = false;
+    for (int s = 0; s < nctx; s++) any_sssp |= owner[s] && searching[s];
     const bool prof = eng->cfg.profile_kernels != 0;
     const bool graphs_on = eng->cfg.use_graphs && !prof;
     for (;;) {
       int levels = 0;
       if (graphs_on) {
         cudaGraphExec_t ex;
-        gst_status s = loop_graph(rwm, &ex);
+        gst_status s = loop_graph(rwm, any_sssp, &ex);
         if (s != GST_OK) return s;
         const uint32_t iters = max_levels > 0 ? (uint32_t)max_levels : 4096u;
         loop_init[0] = iters;
-        loop_init[1] = 0u;
-        CK(cudaMemcpyAsync(d_loop, loop_init, 2 * sizeof(uint32_t), cudaMemcpyHostToDevice,
+        CK(cudaMemcpyAsync(&d_loop->left, loop_init, sizeof(uint32_t), cudaMemcpyHostToDevice,
                            eng->stream));
         CK(cudaGraphLaunch(ex, eng->stream));
-        CK(cudaMemcpyAsync(loop_left, d_loop, sizeof(uint32_t), cudaMemcpyDeviceToHost,
+        CK(cudaMemcpyAsync(loop_left, &d_loop->left, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                            eng->stream));
         levels = (int)iters;
       } else {
         const int ahead = 6;
-        for (int i = 0; i < ahead; i++) launch_level(eng->stream, rwm, any_sssp, prof);
-        cs.launches += (int64_t)ahead * (any_sssp ? 6 : 4);
+        for (int i = 0; i < ahead; i++) launch_level(eng->stream, rwm, any_sssp, prof, nullptr);
+        cs.launches += (int64_t)ahead * (any_sssp ? 4 : 2);
         levels = ahead;
       }
       CK(cudaGetLastError());
@@ -1132,9 +1138,9 @@ struct Runner {
       cs.d2h += (int64_t)sizeof(Ctx) * nctx;
       CK(cudaStreamSynchronize(eng->stream));
       if (graphs_on) {
-        // levels the device loop ran: each is 7 kernels (sssp, rows, grow, 3 ctrl, loop test)
+        // levels the device loop ran: rows and grow each, and sssp and ctrl where needed
         const int64_t ran = (int64_t)levels - (int64_t)loop_left[0];
-        cs.launches += 7 * ran;
+        cs.launches += (any_sssp ? 4 : 2) * ran;
         cs.graph_launches++;
         cs.graph_levels += ran;
         levels = (int)ran;
@@ -1143,7 +1149,8 @@ struct Runner {
       any_sssp = false;
       for (int s = 0; s < nctx; s++) {
         if (!owner[s]) continue;
-        any_sssp |= h_ctx[s].phase == PH_SSSP || h_ctx[s].phase == PH_PREP;
+        searching[s] = h_ctx[s].phase == PH_SSSP || h_ctx[s].phase == PH_PREP;
+        any_sssp |= searching[s];
         any_done |= h_ctx[s].phase >= PH_DONE;
         if (eng->cfg.verbose > 1)
           fprintf(stderr, "[gst run] slot %d k %d phase %u levels %u err %x ub %u n_rows %u in_n %u\n",
@@ -2549,7 +2556,7 @@ gst_status noalloc_solve(int device, cudaStream_t st, int64_t V, int64_t E, cons
   const size_t RW = (size_t)c.RW;
   const int nhb = c.sssp_hops ? hop_budgets(q->hop_bound) : 0;
   const size_t Vs = (size_t)V;
-  size_t off = align256(sizeof(Ctx));
+  size_t off = align256(sizeof(Ctx) + sizeof(LoopCtl));
   auto take = [&](size_t n) {
     const size_t o = off;
     off = align256(off + n);
@@ -2637,6 +2644,7 @@ gst_status noalloc_solve(int device, cudaStream_t st, int64_t V, int64_t E, cons
   c.outcap = kNoallocOutCap;
   c.stackcap = kNoallocStackCap;
   Ctx* d_ctx = (Ctx*)base;
+  LoopCtl* d_loop = (LoopCtl*)(d_ctx + 1);
   NCK(cudaEventRecord(nd->ev[0], st));
   // clear what must start empty (the array keeps the previous call's contents), then
   // upload the context
@@ -2646,23 +2654,22 @@ gst_status noalloc_solve(int device, cudaStream_t st, int64_t V, int64_t E, cons
   NCK(cudaMemsetAsync(c.fm[0], 0, fm_bytes(V), st));
   NCK(cudaMemsetAsync(c.fm[1], 0, fm_bytes(V), st));
   if (nhb) NCK(cudaMemsetAsync(c.dist_h, 0xFF, (size_t)nhb * Vs * ds * 4, st));
+  NCK(cudaMemsetAsync(d_loop, 0, sizeof(LoopCtl), st));
   NCK(cudaMemcpyAsync(d_ctx, &c, sizeof(Ctx), cudaMemcpyHostToDevice, st));
   // the caller's edges are sorted by neighbour only: no light-edge index
   DevGraph G{V, E, d_beg, (const int2*)d_edges, (const int2*)d_edges, nullptr, 0u};
   k_init<<<dim3(8, 1, KMAX), 256, 0, st>>>(d_ctx, nullptr, 1, G, d_grp_ptr, d_members);
-  k_ctrl<<<1, 32, 0, st>>>(d_ctx, nullptr, 1, CTRL_SSSP, 0);
+  k_ctrl<<<1, 32, 0, st>>>(d_ctx, nullptr, 1, 0);
   const size_t smem = rows_smem_per_warp((int)RW) * (size_t)warps;
   int64_t launches = 2;
   Ctx h;
   for (;;) {
     for (int i = 0; i < 6; i++) {
       k_sssp<<<nd->sssp_blocks, 256, 0, st>>>(d_ctx, 1, G, split);
-      k_ctrl<<<1, 128, 0, st>>>(d_ctx, nullptr, 1, CTRL_SSSP, 0);
-      k_rows<<<nd->sms * 4, warps * 32, smem, st>>>(d_ctx, 1, G, split, (int)RW);
-      k_ctrl<<<1, 128, 0, st>>>(d_ctx, nullptr, 1, CTRL_DP_ROWS, 0);
-      k_grow<<<nd->grow_blocks, 256, 0, st>>>(d_ctx, 1, G, split);
-      k_ctrl<<<1, 128, 0, st>>>(d_ctx, nullptr, 1, CTRL_DP_GROW, 0);
-      launches += 6;
+      k_ctrl<<<1, 128, 0, st>>>(d_ctx, nullptr, 1, 0);
+      k_rows<<<nd->sms * 4, warps * 32, smem, st>>>(d_ctx, 1, G, (int)RW, d_loop);
+      k_grow<<<nd->grow_blocks, 256, 0, st>>>(d_ctx, 1, G, split, d_loop, cudaGraphConditionalHandle{}, 0);
+      launches += 4;
     }
     NCK(cudaGetLastError());
     NCK(cudaMemcpyAsync(&h, d_ctx, sizeof(Ctx), cudaMemcpyDeviceToHost, st));
