@@ -1336,15 +1336,23 @@ __global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G
 }
 
 // ---- DP rows step: merge closure of dirty rows in shared memory -------------------
-// Per-warp shared memory: RW cells, RW/32 pending words, RW/32 processed words, three
-// lists of RW cell indices (pending cells, finite cells, the cells of a round),
+// Per-warp shared memory: RW cells, the bounds of up to 31 heights, RW/32 pending words,
+// three lists of RW cell indices (pending cells, finite cells, the cells of a round),
 // 16-B aligned.
 __host__ __device__ __forceinline__ size_t rows_smem_per_warp(int rw_max) {
-  const size_t b = (size_t)rw_max * 8 + (size_t)((rw_max + 31) / 32) * 8 + (size_t)rw_max * 6;
+  const int heights = rw_max / 2 < 31 ? (rw_max / 2 > 0 ? rw_max / 2 : 1) : 31;
+  const size_t b = (size_t)rw_max * 8 + (size_t)heights * KMAX * 4 + (size_t)((rw_max + 31) / 32) * 4 +
+                   (size_t)rw_max * 6;
   return (b + 15) & ~(size_t)15;
 }
 
-// Dynamic shared memory per warp: RWmax cells + RWmax/32 pending words + RWmax list.
+// The kernel is bound by instruction issue (47 % of the warps active, 17-19 lanes a warp), and
+// a row has few changed cells among its 2^k x (D + 1): everything after the closure runs over
+// the list of changed cells, not over the row, and the tour bound takes eight lanes per cell;
+// the rounds come from a mask of the classes that have pending cells.  Before, with passes
+// over the row, a scan for the smallest class per round and one lane per cell in the tour
+// bound: 12.3 to 7.6 ms for 32 queries of k = 5/7 over 141k vertices, 27.7 to 19.1 ms for the
+// 4M-vertex batch.
 // The last block runs the control step of every query.
 __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G, int rw_max,
                                               LoopCtl* lc) {
@@ -1357,12 +1365,12 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
   const size_t per_warp = rows_smem_per_warp(rw_max);
   unsigned char* wbase = s_dyn + per_warp * wib;
   unsigned long long* buf = (unsigned long long*)wbase;
-  uint32_t* pend = (uint32_t*)(wbase + (size_t)rw_max * 8);
-  uint32_t* done = pend + (rw_max + 31) / 32;
-  uint16_t* plist = (uint16_t*)(done + (rw_max + 31) / 32);
+  uint32_t* sb = (uint32_t*)(wbase + (size_t)rw_max * 8);  // the tests' bounds, KMAX per height
+  const int heights = rw_max / 2 < 31 ? (rw_max / 2 > 0 ? rw_max / 2 : 1) : 31;
+  uint32_t* pend = sb + heights * KMAX;
+  uint16_t* plist = (uint16_t*)(pend + (rw_max + 31) / 32);
   uint16_t* flist = plist + rw_max;
   uint16_t* clist = flist + rw_max;
-  uint16_t* list = plist;  // reused for the tour-bound candidates after the closure
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int st_q = -1;
@@ -1392,6 +1400,7 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
     }
     // load the row; list its pending cells (plist) and its finite cells (flist)
     int np = 0, nf = 0;
+    uint32_t classes = 0;  // popcount classes with pending cells, below the full set
     for (int i0 = 0; i0 < RW; i0 += 32) {
       const int i = i0 + lane;
       uint64_t x = CELL_INF;
@@ -1410,47 +1419,34 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
       if (fl) flist[nf + __popc(bf & lt)] = (uint16_t)i;
       np += __popc(bp);
       nf += __popc(bf);
-      if (lane == 0) {
-        pend[i0 >> 5] = bp;
-        done[i0 >> 5] = 0u;
-      }
+      if (pn) classes |= 1u << __popc((uint32_t)i & full);
+      if (lane == 0) pend[i0 >> 5] = bp;
     }
+    classes = __reduce_or_sync(0xffffffffu, classes) & ((1u << k) - 1u);
     if (lane == 0) atomicAnd(&c->rowbits[v >> 5], ~(1u << (v & 31)));
     __syncwarp();
     const uint32_t ubm = hop ? c->ub_cell : c->ub;
     const uint32_t* rest = c->use_tour ? rest_bounds(c) : nullptr;
     // Merge closure T(v, X|Y) <= T(v, X) + T(v, Y), by rounds of popcount class: in a
-    // round the unprocessed pending cells X of the smallest class (clist) are merged
+    // round the pending cells X of the smallest class left (clist) are merged
     // with every finite cell Y disjoint from them, all pairs of the round spread
     // over the lanes (partners from flist, or the submasks of ~X when flist is the
     // longer).  Merges only create cells of a larger class, so a cell is final when
     // its round comes; the cells a round creates or improves join plist (and flist).
-    for (;;) {
-      uint32_t mc = 0xFFFFFFFFu;
-      for (int t = lane; t < np; t += 32) {
-        const uint32_t cc = plist[t];
-        if (!((done[cc >> 5] >> (cc & 31)) & 1u)) mc = min(mc, (uint32_t)__popc(cc & full));
-      }
-      mc = __reduce_min_sync(0xffffffffu, mc);
-      if (mc >= (uint32_t)k) break;  // nothing left below the full set
+    if (nf < 2) classes = 0u;  // nothing to merge with
+    while (classes) {
+      const uint32_t mc = (uint32_t)__ffs(classes) - 1u;
+      classes &= classes - 1u;
       int nl = 0;
       for (int t0 = 0; t0 < np; t0 += 32) {
         const int t = t0 + lane;
-        uint32_t cc = 0;
-        bool sel = false;
-        if (t < np) {
-          cc = plist[t];
-          sel = !((done[cc >> 5] >> (cc & 31)) & 1u) && (uint32_t)__popc(cc & full) == mc;
-        }
+        const uint32_t cc = t < np ? plist[t] : 0u;
+        const bool sel = t < np && (uint32_t)__popc(cc & full) == mc;
         const uint32_t bs = __ballot_sync(0xffffffffu, sel);
         if (sel) clist[nl + __popc(bs & ((1u << lane) - 1u))] = (uint16_t)cc;
         nl += __popc(bs);
       }
       __syncwarp();
-      for (int t = lane; t < nl; t += 32) {
-        const uint32_t cc = clist[t];
-        atomicOr(&done[cc >> 5], 1u << (cc & 31));
-      }
       const uint32_t m = (1u << (k - (int)mc)) - 1u;  // non-empty submasks of ~X
       const bool scan_f = (uint32_t)nf <= m * (uint32_t)DD;
       const uint32_t per = scan_f ? (uint32_t)nf : m * (uint32_t)DD;
@@ -1510,6 +1506,8 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
         if (newf) flist[nf + __popc(bf & lt)] = (uint16_t)tgt;
         np += __popc(bp);
         nf += __popc(bf);
+        // (a merge's class is above the round's: its round is still to come)
+        classes |= __reduce_or_sync(0xffffffffu, newp ? 1u << __popc(tgt & full) : 0u) & ((1u << k) - 1u);
       }
       __syncwarp();
     }
@@ -1540,29 +1538,26 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
         for (int i = 0; i < KMAX; i++) hb[i] = min(e[i], lim);
       }
     }
+    if (lane < (budgets ? DD : 1)) {
+#pragma unroll
+      for (int i = 0; i < KMAX; i++) sb[lane * KMAX + i] = hb[i];
+    }
+    __syncwarp();
     const int64_t deg = G.beg[v + 1] - G.beg[v];
     const int use_tour = c->use_tour;
-    // settle changed states (lane-parallel): write them back, update the full-set
-    // bounds, and apply the one-label and hop tests.  pend keeps the states that
-    // pass; those that still need the tour bound are listed for the warp below.
+    // settle the changed states: write them back, update the full-set bounds, and apply the
+    // one-label and hop tests; clist takes the states that pass
     int ncand = 0;
-    for (int i0 = 0; i0 < RW; i0 += 32) {
-      const int i = i0 + lane;
-      bool keep = false, cand = false;
-      uint32_t dl[KMAX];
-      if (budgets) {
-        const int src = (i < RW ? i : 0) >> k;  // the lane holding this height's bounds
-#pragma unroll
-        for (int b = 0; b < KMAX; b++) dl[b] = __shfl_sync(0xffffffffu, hb[b], src);
-      } else {
-#pragma unroll
-        for (int b = 0; b < KMAX; b++) dl[b] = hb[b];
-      }
-      if (i < RW && ((pend[i >> 5] >> (i & 31)) & 1u)) {
-        const uint64_t x = B((uint32_t)i);
+    for (int t0 = 0; t0 < np; t0 += 32) {
+      const int t = t0 + lane;
+      bool keep = false;
+      uint32_t i = 0;
+      if (t < np) {
+        i = plist[t];
+        const uint64_t x = B(i);
         row[i] = x & ~(uint64_t)PEND;
         const uint32_t cst = cost_of(x);
-        const uint32_t p = (uint32_t)i & full, d = (uint32_t)i >> k;
+        const uint32_t p = i & full, d = i >> k;
         if (p == full) {
           atomicMin(&c->best, ((unsigned long long)cst << 32) | ((unsigned long long)d << 27) | v);
           atomicMin(&c->ub_cell, cst);
@@ -1571,6 +1566,7 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
           uint32_t lb = 0;
           uint64_t one = cst;
           if (c->use_lb) {
+            const uint32_t* dl = sb + (budgets ? d : 0u) * KMAX;
 #pragma unroll
             for (int b = 0; b < KMAX; b++)
               if (b < k && !((p >> b) & 1u)) {
@@ -1582,133 +1578,91 @@ __global__ void __launch_bounds__(256, 4) k_rows(Ctx* ctxs, int nctx, DevGraph G
           const uint32_t bound = hop ? c->ub_cell : c->ub;
           bool grow = 2ull * cst <= (uint64_t)bound && (uint64_t)cst + lb <= (uint64_t)bound;
           if (hop) grow = grow && (int)d < D && cst < bound;
-          if (grow && deg > 0) {
-            keep = true;
-            cand = use_tour != 0;
-          }
+          keep = grow && deg > 0;
         }
       }
       const uint32_t bk = __ballot_sync(0xffffffffu, keep);
-      const uint32_t bc = __ballot_sync(0xffffffffu, cand);
-      if (cand) list[ncand + __popc(bc & ((1u << lane) - 1u))] = (uint16_t)i;
-      ncand += __popc(bc);
-      if (lane == 0) pend[i0 >> 5] = bk;
+      if (keep) clist[ncand + __popc(bk & ((1u << lane) - 1u))] = (uint16_t)i;
+      ncand += __popc(bk);
     }
     __syncwarp();
-    if (ncand > 0) {
+    if (use_tour && ncand > 0) {
       // tour bound of PrunedDP++ (code/PrunedDP++/include/CPUNONHOP.h:433-493): the
       // rest of the tree, doubled, is a closed walk from v through every group of
       // Xb = full \ p, so twice its cost is at least
       //   lb2 = max_a d_a(v) + min_b P(a,b,Xb) + min_b d_b(v)    and
       //   lb1 = min_{a,b} d_a(v) + P(a,b,Xb) + d_b(v),
-      // P = cheapest group sequence from a to b visiting each group of Xb once.
-      // One candidate per lane: the O(k) bound first, the O(k^2) one for the
-      // candidates it keeps (the test is cost + ceil(max(lb1, lb2) / 2) > bound).
+      // P = cheapest group sequence from a to b visiting each group of Xb once (the test is
+      // cost + ceil(max(lb1, lb2) / 2) > bound).  Eight lanes per state, one per group a.
       const uint32_t bound = hop ? __ldcg(&c->ub_cell) : __ldcg(&c->ub);
       const uint32_t* tour = c->tour;
-      const uint32_t Wq = (uint32_t)c->W;
-      for (int t0 = 0; t0 < ncand; t0 += 32) {
-        const int t = t0 + lane;
-        uint32_t dl[KMAX];
-        if (budgets) {
-          const int src = t < ncand ? (int)(list[t] >> k) : 0;
+      const uint32_t* W2s = tour + (size_t)c->W * TOUR_STRIDE;
+      const int ga = lane & 7;
+      int left = 0;
+      for (int t0 = 0; t0 < ncand; t0 += 4) {
+        const int t = t0 + (lane >> 3);
+        const uint32_t i = t < ncand ? clist[t] : 0u;
+        const uint32_t Xb = t < ncand ? full ^ (i & full) : 0u;
+        const bool mine = (Xb >> ga) & 1u;
+        const uint32_t* dl = sb + (budgets ? i >> k : 0u) * KMAX;
+        const uint32_t da = mine ? dl[ga] : COST_INF;
+        uint32_t mind = da;
 #pragma unroll
-          for (int b = 0; b < KMAX; b++) dl[b] = __shfl_sync(0xffffffffu, hb[b], src);
-        } else {
+        for (int o = 1; o < 8; o <<= 1) mind = min(mind, __shfl_xor_sync(0xffffffffu, mind, o));
+        uint64_t t2 = 0, t1 = COST_INF;
+        if (mine) {
+          t2 = (uint64_t)da + __ldg(&W2s[Xb * KMAX + ga]) + mind;
+          const uint4* Wt = (const uint4*)&tour[(size_t)Xb * TOUR_STRIDE + ga * KMAX];
+          const uint4 wa = __ldg(Wt), wb = __ldg(Wt + 1);
+          const uint32_t w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
 #pragma unroll
-          for (int b = 0; b < KMAX; b++) dl[b] = hb[b];
+          for (int b = 0; b < KMAX; b++)
+            if ((Xb >> b) & 1u) t1 = min(t1, (uint64_t)da + w[b] + dl[b]);
         }
-        if (t < ncand) {
-          const uint32_t i = list[t];
-          const uint32_t p = i & full, cst = cost_of(B(i));
-          const uint32_t Xb = full ^ p;
-          const uint32_t* W2 = tour + (size_t)Wq * TOUR_STRIDE + (size_t)Xb * KMAX;
-          uint32_t mind = COST_INF;
+        // both bounds saturate at COST_INF (an unreachable group)
+        uint32_t lb2 = (uint32_t)min(t2, (uint64_t)COST_INF), lb1 = (uint32_t)t1;
 #pragma unroll
-          for (int b2 = 0; b2 < KMAX; b2++)
-            if (b2 < k && ((Xb >> b2) & 1u)) mind = min(mind, dl[b2]);
-          uint64_t lb2 = 0;
-#pragma unroll
-          for (int b2 = 0; b2 < KMAX; b2++)
-            if (b2 < k && ((Xb >> b2) & 1u)) {
-              const uint64_t t2 = (uint64_t)dl[b2] + __ldg(&W2[b2]) + mind;
-              lb2 = t2 > lb2 ? t2 : lb2;
-            }
-          // both bounds saturate at COST_INF (an unreachable group)
-          lb2 = lb2 < COST_INF ? lb2 : COST_INF;
-          bool drop = (uint64_t)cst + (lb2 + 1) / 2 > (uint64_t)bound;
-          if (!drop) {
-            const uint32_t* Wt = tour + (size_t)Xb * TOUR_STRIDE;
-            uint64_t lb1 = ~0ull;
-#pragma unroll
-            for (int a1 = 0; a1 < KMAX; a1++)
-              if (a1 < k && ((Xb >> a1) & 1u)) {
-#pragma unroll
-                for (int b1 = 0; b1 < KMAX; b1++)
-                  if (b1 < k && ((Xb >> b1) & 1u)) {
-                    const uint64_t t1 =
-                        (uint64_t)dl[a1] + __ldg(&Wt[a1 * KMAX + b1]) + dl[b1];
-                    lb1 = t1 < lb1 ? t1 : lb1;
-                  }
-              }
-            lb1 = lb1 < COST_INF ? lb1 : COST_INF;
-            drop = (uint64_t)cst + (lb1 + 1) / 2 > (uint64_t)bound;
-          }
-          if (drop) atomicAnd(&pend[i >> 5], ~(1u << (i & 31)));
+        for (int o = 1; o < 8; o <<= 1) {
+          lb2 = max(lb2, __shfl_xor_sync(0xffffffffu, lb2, o));
+          lb1 = min(lb1, __shfl_xor_sync(0xffffffffu, lb1, o));
         }
+        const uint64_t lb = max(lb1, lb2);
+        const bool stay = t < ncand && ga == 0 && (uint64_t)cost_of(B(i)) + (lb + 1) / 2 <= (uint64_t)bound;
+        const uint32_t bs = __ballot_sync(0xffffffffu, stay);
+        if (stay) clist[left + __popc(bs & ((1u << lane) - 1u))] = (uint16_t)i;
+        left += __popc(bs);
+        __syncwarp();
       }
-      __syncwarp();
+      ncand = left;
     }
     // emit the growing states, each relaxed from its lightest edge on (which lands
-    // at cst + 1 or later): one reservation per list for the whole row
-    {
-      const uint32_t bend = c->bucket_end;
-      uint32_t cn = 0, cf = 0, kmin = COST_INF;
-      for (int i0 = 0; i0 < RW; i0 += 32) {
-        const int i = i0 + lane;
-        if (i < RW && ((pend[i >> 5] >> (i & 31)) & 1u)) {
-          const uint32_t key = cost_of(B(i)) + 1u;
-          if (key >= bend) {
-            cf++;
-            kmin = min(kmin, key);
-          } else {
-            cn++;
-          }
+    // at cst + 1 or later): one reservation per list for 32 of them
+    const uint32_t bend = c->bucket_end;
+    for (int t0 = 0; t0 < ncand; t0 += 32) {
+      const int t = t0 + lane;
+      const uint32_t i = t < ncand ? clist[t] : 0u;
+      const uint32_t cst = t < ncand ? cost_of(B(i)) : 0u;
+      const bool far = t < ncand && cst + 1u >= bend, near = t < ncand && !far;
+      const uint32_t bn = __ballot_sync(0xffffffffu, near), bf = __ballot_sync(0xffffffffu, far);
+      const uint32_t kmin = __reduce_min_sync(0xffffffffu, far ? cst + 1u : COST_INF);
+      uint32_t an = 0, af = 0;
+      if (lane == 0) {
+        if (bn) an = atomicAdd(&c->n_q[c->no], (uint32_t)__popc(bn));
+        if (bf) {
+          af = atomicAdd(&c->n_far[c->f], (uint32_t)__popc(bf));
+          atomicMin(&c->far_min, kmin);
         }
       }
-      const uint32_t sn = warp_incl_scan(cn), sf = warp_incl_scan(cf);
-      const uint32_t tn = __shfl_sync(0xffffffffu, sn, 31), tf = __shfl_sync(0xffffffffu, sf, 31);
-      kmin = __reduce_min_sync(0xffffffffu, kmin);
-      if (tn + tf > 0) {
-        uint32_t bn = 0, bfr = 0;
-        if (lane == 0) {
-          if (tn) bn = atomicAdd(&c->n_q[c->no], tn);
-          if (tf) {
-            bfr = atomicAdd(&c->n_far[c->f], tf);
-            atomicMin(&c->far_min, kmin);
-          }
-        }
-        bn = __shfl_sync(0xffffffffu, bn, 0) + sn - cn;
-        bfr = __shfl_sync(0xffffffffu, bfr, 0) + sf - cf;
-        uint4* nl = c->q[c->no];
-        uint4* fl = c->far[c->f];
-        for (int i0 = 0; i0 < RW; i0 += 32) {
-          const int i = i0 + lane;
-          if (i < RW && ((pend[i >> 5] >> (i & 31)) & 1u)) {
-            const uint32_t cst = cost_of(B(i));
-            const uint32_t p = (uint32_t)i & full, d = (uint32_t)i >> k;
-            const uint4 item = make_uint4(v, p | (d << 16), cst, 0u);
-            if (cst + 1u >= bend) {
-              if (bfr < c->farcap) fl[bfr] = item;
-              else atomicOr(&c->error, (uint32_t)ERR_FARCAP);
-              bfr++;
-            } else {
-              if (bn < c->qcap) nl[bn] = item;
-              else atomicOr(&c->error, (uint32_t)ERR_QCAP);
-              bn++;
-            }
-          }
-        }
+      const uint32_t lt = (1u << lane) - 1u;
+      an = __shfl_sync(0xffffffffu, an, 0) + __popc(bn & lt);
+      af = __shfl_sync(0xffffffffu, af, 0) + __popc(bf & lt);
+      const uint4 item = make_uint4(v, (i & full) | ((i >> k) << 16), cst, 0u);
+      if (far) {
+        if (af < c->farcap) c->far[c->f][af] = item;
+        else atomicOr(&c->error, (uint32_t)ERR_FARCAP);
+      } else if (near) {
+        if (an < c->qcap) c->q[c->no][an] = item;
+        else atomicOr(&c->error, (uint32_t)ERR_QCAP);
       }
     }
     // statistics: one atomic per query change of the warp, not per row
