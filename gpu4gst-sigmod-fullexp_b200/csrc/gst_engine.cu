@@ -382,10 +382,12 @@ struct Job {
   uint32_t ds = DIST_STRIDE;     // uint32 per distance row
   uint32_t* cache_dst = nullptr; // a group-cache fill: the distances of group gids[0] to
                                  // every vertex go here (V entries), no DP
-  // batch-shared search: 1 when a shared table of the runner holds this query's distances
-  // (its groups in columns ss_cols), exact up to ss_cut; 2 when its table was given back
-  // before it was admitted (it searches on its own)
+  // batch-shared search: 1 when the shared table ss_id of the runner holds this query's
+  // distances (its groups in columns ss_cols), exact up to ss_cut; 2 when it searches on its
+  // own (no memory for a table, a search that failed, or a table given back before the query
+  // was admitted); 0 before either
   int ss = 0;
+  int ss_id = 0;
   uint16_t ss_cols[KMAX] = {0};
   uint32_t ss_cut = 0;
   std::atomic<bool> done{false};
@@ -451,16 +453,18 @@ struct Runner {
     void* mem = nullptr;
     size_t bytes = 0;
     BsCtx* d_b = nullptr;
-    int remaining = 0;
+    int id = 0;
+    int remaining = 0;               // its queries not admitted yet
     int D = 0;                       // 0: unbounded distances; else the hop bound
     uint32_t Gp = 0;                 // columns of the tables
     uint32_t* tab[KMAX + 1] = {};    // hop-bounded: d^{<=h} tables (device); tab[D] = dist
     uint32_t* dist = nullptr;        // the distance table (device)
   };
-  std::vector<Shared> shs;           // pending shared tables, at most one per kind (D)
-  Shared* shared_of(int D) {
+  std::vector<Shared> shs;           // pending shared tables
+  int last_shared = 0;
+  Shared* shared_of(const Job& j) {
     for (Shared& x : shs)
-      if (x.D == D && x.d_b) return &x;
+      if (j.ss == 1 && x.id == j.ss_id) return &x;
     return nullptr;
   }
 
@@ -752,7 +756,7 @@ struct Runner {
     }
     // a query of the batch-shared search: its distances are in the runner's shared
     // table, exact up to its cutoff; it starts at the bounds pass
-    Shared* S = j->ss == 1 ? shared_of(hop ? q->hop_bound : 0) : nullptr;
+    Shared* S = shared_of(*j);
     if (S) {
       c.cut_fix = std::max(1u, j->ss_cut);
       a.stride = S->Gp;
@@ -840,7 +844,7 @@ struct Runner {
   // of hop bound D (1..KMAX), over their distinct groups `cols` (at most BS_COLS groups,
   // BS_MAXQ queries).  On success every job is marked (ss = 1) with its columns and
   // cutoff; without memory for the tables, or when the search reports an error, the jobs
-  // keep their own searches.
+  // search on their own (ss = 2).
   gst_status shared_search(const std::vector<Job*>& jobs, const std::vector<int32_t>& cols, int D) {
     gst_status s = GST_OK;
     if (n_aq) {  // nothing admitted reads memory that is taken below
@@ -848,6 +852,7 @@ struct Runner {
       if (s != GST_OK) return s;
       CK(cudaStreamSynchronize(eng->stream));  // h_aq is free again
     }
+    for (Job* j : jobs) j->ss = 2;  // until the search has succeeded
     const int64_t V = g->V;
     const uint32_t ncols = (uint32_t)cols.size();
     const uint32_t Gp = (ncols + 7u) / 8u * 8u, Wm = (Gp + 31u) / 32u;
@@ -883,6 +888,7 @@ struct Runner {
     shs.back().mem = p;
     shs.back().bytes = off;
     shs.back().D = D;
+    shs.back().id = ++last_shared;
     BsCtx h;
     memset(&h, 0, sizeof(h));
     h.D = (uint32_t)D;
@@ -991,6 +997,7 @@ struct Runner {
       for (int i = 0; i < KMAX; i++) jobs[q]->ss_cols[i] = i < jobs[q]->q.k ? hb.qcol[q][i] : 0;
       jobs[q]->ss_cut = cut;
       jobs[q]->ss = 1;
+      jobs[q]->ss_id = S.id;
     }
     S.remaining = (int)jobs.size();
     return GST_OK;
@@ -1339,6 +1346,7 @@ struct gst_server {
 
 namespace {
 gst_status maybe_shared_search(Runner& R, std::deque<Job*>& pending);  // with the batch driver
+bool waits_for_search(const Runner& R, const Job* j);
 }  // namespace
 
 namespace {
@@ -1382,6 +1390,8 @@ void server_loop(gst_server* sv) {
           if (sv->pending.empty()) break;
           j = sv->pending.front();
         }
+        // arrived after the search: it waits for the next one, at the next level boundary
+        if (waits_for_search(R, j)) break;
         gst_status s = R.admit(j);
         if (s == GST_NOT_READY) break;
         std::lock_guard<std::mutex> lk(sv->mu);
@@ -1390,6 +1400,7 @@ void server_loop(gst_server* sv) {
           sv->admitted++;
           continue;
         }
+        if (Runner::Shared* S = R.shared_of(*j)) S->remaining--;  // never gathers its columns
         memset(j->out, 0, sizeof(gst_result));
         j->out->status = s;
         j->out->user_tag = j->q.user_tag;
@@ -1397,10 +1408,10 @@ void server_loop(gst_server* sv) {
         sv->completed++;
         sv->cv_done.notify_all();
       }
-      bool waiting;
+      bool waiting;  // an arrival waits for a slot or memory (not for the next search)
       {
         std::lock_guard<std::mutex> lk(sv->mu);
-        waiting = !sv->pending.empty();
+        waiting = !sv->pending.empty() && !waits_for_search(R, sv->pending.front());
       }
       gst_status s = s_pre;
       if (s == GST_OK && R.active == 0 && waiting && !R.shs.empty()) {
@@ -1811,26 +1822,35 @@ gst_status shared_search_kind(Runner& R, std::deque<Job*>& pending, int kind) {
   return R.shared_search(chunk, cols, kind);
 }
 
-// Before admitting: for every kind (unbounded, or one hop bound D) with no shared table
-// pending and an eligible query waiting, search the groups of that kind's first
-// queries together (in order, up to BS_COLS distinct groups and BS_MAXQ queries).  A
-// lone query takes the same path: its search over k columns on these kernels is faster
-// than the per-query group-mask search on large graphs.  Kinds are searched in the
-// order their first queries wait.
+// Before admitting: for every kind (unbounded, or one hop bound D) with an eligible query
+// waiting and fewer searched ones than there are free slots, search the groups of that
+// kind's first queries together (in order, up to BS_COLS distinct groups and BS_MAXQ
+// queries).  A lone query takes the same path: its search over k columns on these kernels
+// is faster than the per-query group-mask search on large graphs.  Kinds are searched in
+// the order their first queries wait.  An eligible query is admitted only once it has been
+// part of a search: with one table per kind, and newcomers admitted on sight, 36 of a batch
+// of 100 queries searched alone, and most of 24 that arrived at a server while it took in
+// the first (90 ms for those over 1M vertices, 32 now; the 100 over 20k 9.5 and 8.8 ms).
 gst_status maybe_shared_search(Runner& R, std::deque<Job*>& pending) {
   if (!R.eng->cfg.batch_search) return GST_OK;
   R.shared_release(false);
   std::vector<int> kinds;
   for (Job* j : pending) {
     const int jk = shared_kind(R, j);
-    if (jk >= 0 && !R.shared_of(jk) && std::find(kinds.begin(), kinds.end(), jk) == kinds.end())
-      kinds.push_back(jk);
+    if (jk < 0 || std::find(kinds.begin(), kinds.end(), jk) != kinds.end()) continue;
+    int searched = 0;
+    for (const Runner::Shared& x : R.shs) searched += x.D == jk ? x.remaining : 0;
+    if (searched < R.max_slots - R.active) kinds.push_back(jk);
   }
   for (int kind : kinds) {
     gst_status s = shared_search_kind(R, pending, kind);
     if (s != GST_OK) return s;
   }
   return GST_OK;
+}
+// Whether job j waits for a shared search to come.
+bool waits_for_search(const Runner& R, const Job* j) {
+  return R.eng->cfg.batch_search && shared_kind(R, j) >= 0;
 }
 
 gst_status drive(Runner& R, std::deque<Job*>& pending, int B) {
@@ -1842,7 +1862,12 @@ gst_status drive(Runner& R, std::deque<Job*>& pending, int B) {
   while (st == GST_OK && (!pending.empty() || R.active > 0)) {
     st = maybe_shared_search(R, pending);
     if (st != GST_OK) break;
+    bool erased = false;
     for (auto it = pending.begin(); it != pending.end() && R.active < R.max_slots;) {
+      if (waits_for_search(R, *it)) {
+        ++it;
+        continue;
+      }
       gst_status s = R.admit(*it);
       if (s == GST_NOT_READY) {
         ++it;
@@ -1850,10 +1875,7 @@ gst_status drive(Runner& R, std::deque<Job*>& pending, int B) {
       }
       if (s == GST_OOM_ADMISSION) {
         Job* j = *it;
-        if (j->ss == 1) {  // never gathers its columns
-          Runner::Shared* S = R.shared_of(j->q.hop_bound < 0 ? 0 : j->q.hop_bound);
-          if (S) S->remaining--;
-        }
+        if (Runner::Shared* S = R.shared_of(*j)) S->remaining--;  // never gathers its columns
         j->out->status = GST_OOM_ADMISSION;
         j->out->user_tag = j->q.user_tag;
         fail(eng, GST_OOM_ADMISSION, "solve: the query's state table does not fit the memory budget");
@@ -1862,6 +1884,7 @@ gst_status drive(Runner& R, std::deque<Job*>& pending, int B) {
         break;
       }
       it = pending.erase(it);
+      erased = true;
     }
     if (st == GST_OK && R.active == 0 && !pending.empty() && !R.shs.empty()) {
       // nothing runs and the shared tables hold memory a waiting query needs: give them
@@ -1870,6 +1893,16 @@ gst_status drive(Runner& R, std::deque<Job*>& pending, int B) {
         if (j->ss == 1) j->ss = 2;
       R.shared_release(true);
       continue;
+    }
+    if (st == GST_OK && R.active == 0 && !pending.empty()) {
+      // nothing runs: go on to the queries that wait for a search, without one if need be
+      bool waiting = false;
+      for (Job* j : pending)
+        if (waits_for_search(R, j)) {
+          waiting = true;
+          if (!erased) j->ss = 2;
+        }
+      if (waiting) continue;
     }
     if (st != GST_OK || R.active == 0) break;
     st = R.run(0);

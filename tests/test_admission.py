@@ -1,7 +1,10 @@
 """Starting queries together (k_admit) and the sizes of their row pools: a tight memory budget
 (a pool of an eighth of the vertices that the heavy queries overflow, then the dense layout),
 a wide one (a mapped pool of up to one row per vertex), and batches whose queries start from a
-shared search, from cached groups, from both and alone, all give the reference's costs."""
+shared search, from cached groups, from both and alone, all give the reference's costs.
+Queries beyond one search's 64 wait for the next search; without memory for a search's table
+they search on their own."""
+import numpy as np
 import pytest
 
 import gst_b200 as G
@@ -44,4 +47,32 @@ def test_mixed_starts_keep_the_optima(search):
             _check(g, grp, q, h, dg.solve(q, h), _ref(w))
         dg.close()
     finally:
+        eng.close()
+
+
+@pytest.mark.parametrize("budget", [0, 60 << 20])
+@pytest.mark.parametrize("slots", [1, 7, 32])
+def test_more_queries_than_one_search(budget, slots):
+    g = G.synth_rmat(30_000, 120_000, 41)
+    grp = G.synth_groups_zipf(g.V, 500, 1.5, 1, 40, 42)
+    rng = np.random.default_rng(43)
+    qs = [rng.choice(500, size=int(rng.integers(2, 5)), replace=False).astype(np.int32) for _ in range(90)]
+    hops = [None if x < 0.5 else int(rng.integers(0, 4)) for x in rng.random(90)]
+    ref = G.Engine(0, batch_search=0)
+    eng = G.Engine(0, max_batch=slots, mem_budget_bytes=budget)
+    try:
+        alone = ref.graph(g, grp)
+        dg = eng.graph(g, grp)
+        want = [(a.status, a.cost) for a in (alone.solve(q, h) for q, h in zip(qs, hops))]
+        got = dg.solve_batch(qs, hops)
+        assert [(a.status, a.cost) for a in got] == want
+        if budget == 0:
+            sv = dg.server()
+            tickets = [sv.submit(q, h) for q, h in zip(qs, hops)]
+            assert [(a.status, a.cost) for a in map(sv.wait, tickets)] == want
+            sv.close()
+        alone.close()
+        dg.close()
+    finally:
+        ref.close()
         eng.close()
