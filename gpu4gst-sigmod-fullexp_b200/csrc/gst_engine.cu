@@ -74,7 +74,8 @@ constexpr size_t kTourWords = ((size_t)1 << KMAX) * (TOUR_STRIDE + KMAX + 1);
 constexpr uint32_t kOutCap = 1u << 16;
 constexpr uint32_t kStackCap = 1u << 18;
 
-constexpr size_t kDenseBytes = (size_t)32 << 20;  // tables laid out densely up to here
+constexpr size_t kDenseBytes = (size_t)32 << 20;  // tables laid out densely up to here,
+constexpr int64_t kDenseVertices = 1 << 17;       // or to here
 constexpr size_t kPoolRoom = (size_t)2 << 30;     // bytes a row pool may take beyond its eighth
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -83,22 +84,25 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // whole 16-byte words.
 size_t fm_bytes(int64_t V) { return ((size_t)V + 15) / 16 * 16; }
 
+// Whether a table of at least V rows is laid out densely (one row per vertex, no map):
+// where it is small or has few vertices (clearing it costs less than the map's extra
+// reads), and after a capacity retry.
+bool dense_rows(int64_t V, size_t rw, uint64_t rows, int boost) {
+  return rows >= (uint64_t)V &&
+         ((size_t)V * rw * 8 <= kDenseBytes || V <= kDenseVertices || boost > 0);
+}
 // Rows of a query's row pool: an eighth of the vertices (at least 64k rows), or as many as
-// `room` bytes hold, four times more per capacity retry, at most one per vertex.  Most
+// `room` bytes hold, four times more per capacity retry; at most 5/4 of the vertices, since
+// every lost race for a row leaves one unused, or one per vertex in the dense layout.  Most
 // queries write rows for a few percent of the vertices (their pruning keeps the DP near the
 // optimal trees), but the heaviest k = 7 ones overflow an eighth and then run twice, the
 // second time with a search of their own (10 to 22 of 155 ms of a batch of 32 over 4M
 // vertices, the lost first run not counted: 129 ms without).
 uint32_t pool_rows(int64_t V, size_t rw, size_t room, int boost) {
   uint64_t r = std::max<uint64_t>(std::max<uint64_t>(1u << 16, (uint64_t)V / 8), room / (rw * 8));
-  for (int i = 0; i < boost; i++) r = std::min<uint64_t>(r * 4, (uint64_t)V);
-  return (uint32_t)std::min<uint64_t>(r, (uint64_t)V);
-}
-// Whether a table of V rows is laid out densely (one row per vertex, no map): where it is
-// small (clearing it costs less than the map's extra reads), and after a capacity retry
-// (a pool of V rows can still run out: a lost race for a row leaves one unused).
-bool dense_rows(int64_t V, size_t rw, uint32_t rows, int boost) {
-  return (int64_t)rows >= V && ((size_t)V * rw * 8 <= kDenseBytes || boost > 0);
+  for (int i = 0; i < boost; i++) r = std::min<uint64_t>(r * 4, 1u << 30);
+  if (dense_rows(V, rw, r, boost)) return (uint32_t)V;
+  return (uint32_t)std::min<uint64_t>(r, (uint64_t)V + (uint64_t)V / 4);
 }
 
 // Lay out (or, with base == nullptr, only size) a slot of V vertices: a row pool of
@@ -770,9 +774,12 @@ struct Runner {
     c.sssp_mask = c.sssp_hops ? 2u : (c.bucket_end == 0xFFFFFFFFu ? 1u : 0u);
     // the pool takes every row the slot's table holds; only the rows the slot's last
     // query wrote need clearing
-    c.pool_cap = (uint32_t)std::min<uint64_t>((uint64_t)g->V, m.table_bytes / ((size_t)c.RW * 8));
+    c.pool_cap = (uint32_t)std::min<uint64_t>(1u << 30, m.table_bytes / ((size_t)c.RW * 8));
     c.pool_n = 0;
-    if (dense_rows(g->V, (size_t)c.RW, c.pool_cap, j->boost)) c.rowmap = nullptr;
+    if (dense_rows(g->V, (size_t)c.RW, c.pool_cap, j->boost)) {
+      c.rowmap = nullptr;
+      c.pool_cap = (uint32_t)g->V;
+    }
     a.dirty16 = (m.table_dirty + 15) / 16;
     m.table_dirty = 0;
     n_aq++;
