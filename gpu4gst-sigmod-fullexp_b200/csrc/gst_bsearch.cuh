@@ -27,8 +27,18 @@
 // row improved in round r-1 (round 0: the members, distance 0) from table r into table
 // r+1 alone.  Table r is final while round r reads it, so no snapshot is needed, and
 // the result is the per-query rounds'.  Stars come from tables r with 2r <= D (trees of
-// diameter <= D), as in the per-query search; after the last round the tables above
-// it are filled from it.
+// diameter <= D), as in the per-query search.
+//
+// The last rounds pull.  Table h bounds the states of height D - h only, and those hang at
+// vertices within D - h edges of their query's members: table D is read at the members
+// themselves, table D-1 at their neighbours.  So the last round (and, from D = 4 on, the
+// one before it) takes each such vertex and the sectors of the queries that may have a state
+// there, and looks at its own edges, instead of pushing along the edges of everything within
+// D - 1 (D - 2) edges of a member, which is the whole graph.  Elsewhere these tables hold
+// upper bounds that no state reads (and are zero at members only, like the others).  The
+// bits to pull at come with the search: the members, and what round 0 announced.
+// 32 queries with D = 3/4/5 over 1M vertices relax 410 M sectors instead of 1303 M (search
+// 15.4 to 6.2 ms), the 4M-vertex batch 3.1 G instead of 5.3 G.
 //
 // Edge classes (unbounded searches): the edges are relaxed light ones first, to a fixpoint,
 // and only then the heavier ones, from every vertex whose distances changed since its
@@ -80,6 +90,10 @@ struct BsCtx {
   uint32_t cut_pm;      // query cutoff: star x cut_pm / 1000
   uint32_t D;           // 0: unbounded distances; else the hop bound (rounds 0..D-1)
   uint32_t round;       // hop-bounded: the current round
+  uint32_t pull;        // hop-bounded: the first round that pulls
+  uint32_t* near[2];    // hop-bounded: V x Wm, columns with a member at the vertex (0), or at
+                        // it or a neighbour (1)
+  uint32_t colsec[BS_COLS];  // per column: the sectors of the queries that use it
   uint32_t* tab[KMAX + 1];  // hop-bounded: tab[h] = d^{<=h} (V x Gp), tab[D] = dist
   uint32_t nq;          // queries
   uint32_t qk[BS_MAXQ];
@@ -110,7 +124,10 @@ __global__ void k_bs_seed(BsCtx* b, DevGraph G, const int64_t* grp_ptr, const in
     const uint32_t v = (uint32_t)members[j];
     if (v >= G.V) continue;
     atomicMin(&(b->D ? b->tab[1] : b->dist)[(uint64_t)v * Gp + c], 0u);
-    if (G.beg[v + 1] > G.beg[v]) atomicOr(&b->fm[b->in][(uint64_t)v * Wm + (c >> 5)], 1u << (c & 31));
+    const uint64_t word = (uint64_t)v * Wm + (c >> 5);
+    if (G.beg[v + 1] > G.beg[v]) atomicOr(&b->fm[b->in][word], 1u << (c & 31));
+    for (int i = 0; i < 2; i++)
+      if (b->near[i]) atomicOr(&b->near[i][word], 1u << (c & 31));
   }
 }
 
@@ -140,19 +157,28 @@ __device__ __forceinline__ void bs_lower_cutoffs(BsCtx* b, uint32_t* s_cut) {
 // (vertex, query).  VPT neighbouring vertices per thread: with four, their words come in
 // Wm 16-byte loads issued together, which is all a step that announces few vertices does
 // (large graphs); with one, the stars of a small graph spread over four times the warps.
-template <int VPT>
-__global__ void __launch_bounds__(256) k_bs_scan(BsCtx* b, DevGraph G) {
+// PULL: a pulling round, whose items are the vertices of near[D - 1 - r] with the sectors of
+// the queries that may have a state there.
+template <int VPT, bool PULL>
+__global__ void __launch_bounds__(256, 4) k_bs_scan(BsCtx* b, DevGraph G) {
   __shared__ uint32_t s_star[BS_MAXQ];
   __shared__ uint32_t s_cut[BS_COLS];
   __shared__ uint16_t s_col[BS_MAXQ][KMAX];
   __shared__ uint32_t s_k[BS_MAXQ];
+  __shared__ uint32_t s_sec[PULL ? BS_COLS : 1];  // colsec
   __shared__ uint32_t s_v[256 / 32][32];  // per warp: the announced vertices
   __shared__ uint32_t s_sum[2][256 / 32], s_work[2][256 / 32], s_base[2];
   if (b->done) return;
   const uint32_t Wm = b->Wm, cls = b->cls, Gp = b->Gp, nq = b->nq, D = b->D, r = b->round;
   const uint32_t chunk = b->chunk, cap = b->item_cap;
-  uint32_t* from = cls ? b->later : b->fm[b->in];
-  uint32_t* later = cls + 1u < b->ncls ? b->later : nullptr;
+  const bool two = b->ncls > 1u;
+  uint32_t* from = PULL ? b->near[D - 1u - r] : cls ? b->later : b->fm[b->in];
+  // where the announced columns are kept for later: a light step's for the heavy class, what
+  // round 0 of a hop-bounded search announced for the round that pulls at the neighbours
+  uint32_t* keep = D ? (r == 1u ? b->near[1] : nullptr) : two && cls == 0u ? b->later : nullptr;
+  uint32_t* am = b->am;
+  uint2* items = b->items;
+  const uint32_t* cend = b->cend;
   // Every improved distance is announced to the light class, and on to the heavy one.  With
   // two classes the light scans, of which there are many, look for stars only at the
   // vertices of highest degree (the lowest ids), where the best ones are, and the heavy
@@ -160,6 +186,8 @@ __global__ void __launch_bounds__(256) k_bs_scan(BsCtx* b, DevGraph G) {
   const bool stars = D == 0u || (r >= 1u && 2u * r <= D);
   const int64_t star_end = !D && cls == 0u && b->ncls > 1u ? (G.V + 15) / 16 : G.V;
   const uint32_t* tab = D ? b->tab[r] : b->dist;
+  if constexpr (PULL)
+    for (uint32_t c = threadIdx.x; c < BS_COLS; c += blockDim.x) s_sec[c] = b->colsec[c];
   for (uint32_t q = threadIdx.x; q < BS_MAXQ; q += blockDim.x) {
     s_star[q] = COST_INF;
     s_k[q] = q < nq ? b->qk[q] : 0u;
@@ -174,37 +202,101 @@ __global__ void __launch_bounds__(256) k_bs_scan(BsCtx* b, DevGraph G) {
        base += (int64_t)gridDim.x * blockDim.x) {
     const int64_t first = (base + threadIdx.x) * VPT;
     uint32_t hit = 0;  // bit i: vertex first + i is announced
+    uint32_t cnt = 0;  // its active sectors, in byte i
+    // (loads before stores throughout: the stores may alias them for the compiler, and one
+    // access after the other made a scan of 4.6M announced vertices 1.1 ms long, 0.15 now)
     if (base + threadIdx.x < spans) {
-      if (VPT == 4) {
-        const uint4* p = (const uint4*)(from + first * Wm);
-        for (uint32_t w = 0; w < Wm; w++) {  // its word 4 w + i is vertex first + (4 w + i) / Wm's
-          const uint4 x = p[w];  // (a cached load: a line serves several of them)
-          hit |= (x.x ? 1u << (4 * w) / Wm : 0u) | (x.y ? 1u << (4 * w + 1) / Wm : 0u) |
-                 (x.z ? 1u << (4 * w + 2) / Wm : 0u) | (x.w ? 1u << (4 * w + 3) / Wm : 0u);
+      if constexpr (PULL) {
+        for (int i = 0; i < VPT; i++) {
+          uint32_t needed = 0;
+          if (first + i < G.V)
+            for (uint32_t w = 0; w < Wm; w++)
+              for (uint32_t x = __ldcg(&from[(first + i) * Wm + w]); x; x &= x - 1u)
+                needed |= s_sec[w * 32u + (uint32_t)__ffs(x) - 1u];
+          if (!needed) continue;
+          hit |= 1u << i;
+          cnt |= (uint32_t)__popc(needed) << (8 * i);
+          for (uint32_t w = 0; w < Wm; w++) {  // the needed sectors, all their columns
+            const uint32_t x = (needed >> (4u * w)) & 0xFu;
+            am[(first + i) * Wm + w] = ((x & 1u) | (x & 2u) << 7 | (x & 4u) << 14 | (x & 8u) << 21) * 0xFFu;
+          }
+        }
+      } else if constexpr (VPT == 4) {
+        uint4* f4 = (uint4*)(from + first * Wm);
+        uint4* a4 = (uint4*)(am + first * Wm);
+        uint4* k4 = keep ? (uint4*)(keep + first * Wm) : nullptr;
+        uint32_t some = 0;
+        for (uint32_t w = 0; w < Wm; w++) {  // (cached loads: a line serves several of them)
+          const uint4 x = f4[w];
+          some |= x.x | x.y | x.z | x.w;
+        }
+        for (uint32_t w0 = 0; some && w0 < Wm; w0 += 4) {
+          uint4 x[4], y[4];
+          bool on[4];
+#pragma unroll
+          for (uint32_t j = 0; j < 4; j++)
+            x[j] = w0 + j < Wm ? f4[w0 + j] : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+          for (uint32_t j = 0; j < 4; j++) {
+            on[j] = (x[j].x | x[j].y | x[j].z | x[j].w) != 0u;
+            y[j] = on[j] && k4 ? k4[w0 + j] : make_uint4(0u, 0u, 0u, 0u);
+          }
+#pragma unroll
+          for (uint32_t j = 0; j < 4; j++) {
+            if (w0 + j < Wm) a4[w0 + j] = x[j];
+            if (!on[j]) continue;
+            f4[w0 + j] = make_uint4(0u, 0u, 0u, 0u);
+            if (k4) k4[w0 + j] = make_uint4(x[j].x | y[j].x, x[j].y | y[j].y, x[j].z | y[j].z, x[j].w | y[j].w);
+            const uint32_t c[4] = {x[j].x, x[j].y, x[j].z, x[j].w};
+#pragma unroll
+            for (uint32_t i = 0; i < 4; i++) {
+              const uint32_t at = (4u * (w0 + j) + i) / Wm;  // the word's vertex
+              const uint32_t n = ((c[i] & 0xFFu) != 0u) + ((c[i] & 0xFF00u) != 0u) +
+                                 ((c[i] & 0xFF0000u) != 0u) + (c[i] >> 24 != 0u);
+              hit |= (c[i] != 0u) << at;
+              cnt += n << (8u * at);
+            }
+          }
         }
       } else {
-        for (uint32_t w = 0; w < Wm; w++) hit |= __ldcg(&from[first * Wm + w]) ? 1u : 0u;
+        uint32_t x[BS_COLS / 32], y[BS_COLS / 32];
+#pragma unroll
+        for (uint32_t w = 0; w < BS_COLS / 32; w++) {
+          x[w] = w < Wm ? __ldcg(&from[first * Wm + w]) : 0u;
+          hit |= x[w] != 0u;
+        }
+        if (hit) {
+#pragma unroll
+          for (uint32_t w = 0; w < BS_COLS / 32; w++) y[w] = keep && w < Wm ? keep[first * Wm + w] : 0u;
+#pragma unroll
+          for (uint32_t w = 0; w < BS_COLS / 32; w++)
+            if (w < Wm) {
+              am[first * Wm + w] = x[w];
+              from[first * Wm + w] = 0u;
+              if (keep) keep[first * Wm + w] = x[w] | y[w];
+              cnt += ((x[w] & 0xFFu) != 0u) + ((x[w] & 0xFF00u) != 0u) + ((x[w] & 0xFF0000u) != 0u) +
+                     (x[w] >> 24 != 0u);
+            }
+        }
       }
     }
     if (!__syncthreads_or(hit != 0u)) continue;
+    more |= hit && two && cls == 0u;
     uint32_t whole[VPT], rest[VPT], nw = 0, nr = 0, ww = 0, wr = 0;
+    int64_t bg[VPT + 1];
+    uint32_t light[VPT];
+    if (hit) {
+#pragma unroll
+      for (int i = 0; i <= VPT; i++) bg[i] = first + i <= G.V ? G.beg[first + i] : 0;
+#pragma unroll
+      for (int i = 0; i < VPT; i++) light[i] = two && first + i < G.V ? __ldg(&cend[first + i]) : 0u;
+    }
 #pragma unroll
     for (int i = 0; i < VPT; i++) {
       whole[i] = rest[i] = 0u;
       if (!((hit >> i) & 1u)) continue;
-      const uint32_t v = (uint32_t)(first + i);
-      uint32_t sectors = 0;
-      for (uint32_t w = 0; w < Wm; w++) {
-        const uint32_t x = __ldcg(&from[(uint64_t)v * Wm + w]);
-        b->am[(uint64_t)v * Wm + w] = x;
-        from[(uint64_t)v * Wm + w] = 0u;
-        if (later && x) later[(uint64_t)v * Wm + w] |= x;
-        sectors += ((x & 0xFFu) != 0u) + ((x & 0xFF00u) != 0u) + ((x & 0xFF0000u) != 0u) + (x >> 24 != 0u);
-      }
-      more |= later != nullptr;
-      int64_t lo, hi;
-      class_range(b, cls, v, G.beg[v + 1] - G.beg[v], &lo, &hi);
-      const uint32_t edges = (uint32_t)(hi - lo);
+      const uint32_t deg = (uint32_t)(bg[i + 1] - bg[i]), sectors = (cnt >> (8 * i)) & 0xFFu;
+      const uint32_t edges = !two ? deg : cls ? deg - light[i] : light[i];
       whole[i] = edges / chunk;
       rest[i] = edges % chunk != 0u;
       nw += whole[i];
@@ -249,14 +341,14 @@ __global__ void __launch_bounds__(256) k_bs_scan(BsCtx* b, DevGraph G) {
         const uint32_t n = __shfl_sync(0xffffffffu, whole[i], src), t = __shfl_sync(0xffffffffu, tw, src);
         const uint32_t v = __shfl_sync(0xffffffffu, (uint32_t)(first + i), src);
         for (uint32_t j = (uint32_t)lane; j < n; j += 32)
-          if (t + j < cap) b->items[t + j] = make_uint2(v, j);
+          if (t + j < cap) items[t + j] = make_uint2(v, j);
       }
       if (whole[i] <= 16u)
         for (uint32_t j = 0; j < whole[i]; j++)
-          if (tw + j < cap) b->items[tw + j] = make_uint2((uint32_t)(first + i), j);
+          if (tw + j < cap) items[tw + j] = make_uint2((uint32_t)(first + i), j);
       tw += whole[i];
       if (rest[i]) {
-        if (tr < cap) b->items[cap - 1u - tr] = make_uint2((uint32_t)(first + i), whole[i]);
+        if (tr < cap) items[cap - 1u - tr] = make_uint2((uint32_t)(first + i), whole[i]);
         tr++;
       }
     }
@@ -287,10 +379,10 @@ __global__ void __launch_bounds__(256) k_bs_scan(BsCtx* b, DevGraph G) {
 }
 
 // The next step (the last block of a relax launch): announced vertices first, else the
-// heavy edges that wait; without any the search is done.
+// heavy edges that wait; without any the search is done.  Hop-bounded: D rounds.
 __device__ __forceinline__ void bs_advance(BsCtx* b) {
-  const uint32_t cls = __ldcg(&b->ann) ? 0u : 1u;
-  if (__ldcg(&b->error) || (cls && !__ldcg(&b->have))) {
+  const uint32_t cls = b->D || __ldcg(&b->ann) ? 0u : 1u;
+  if (__ldcg(&b->error) || (b->D ? b->round + 1u >= b->D : cls && !__ldcg(&b->have))) {
     b->done = 1u;
   } else if (++b->steps > b->max_steps) {
     b->error |= BS_ERR_STEPS;
@@ -327,9 +419,11 @@ constexpr int BS_U = 2;        // (edge, sector) pairs per lane in flight
 constexpr uint32_t BS_TAKE = 1024;  // pairs per take, about
 constexpr uint32_t BS_LIST = 256;   // units per take, at most
 struct __align__(16) BsUnit {  // one unit of a window
-  int nd[8];                   // -distance per column (inactive: -INT_MAX)
+  int nd[8];                   // -distance per column (inactive: -INT_MAX); pulling: the
+                               // target's distances, at most cutoff + 1
   uint32_t sec;                // the sector
-  uint32_t pad[3];             // 48-byte stride: eight lanes' 16-byte loads hit 32 banks
+  uint32_t at;                 // pulling: the target's row, in sectors
+  uint32_t pad[2];             // 48-byte stride: eight lanes' 16-byte loads hit 32 banks
 };
 struct __align__(16) BsWork {  // one item of a window with work
   int64_t eb;                  // its first edge
@@ -337,6 +431,8 @@ struct __align__(16) BsWork {  // one item of a window with work
   uint32_t unit;               // its first unit | its units c << 5 | ceil(2^16 / c) << 11: a
                                // pair's edge is (pair * that) >> 16, exact below 2^11 pairs
 };
+// PULL: the items are targets; a pair reads the neighbour's row and lowers the item's.
+template <bool PULL>
 __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G) {
   // (shared memory is kept small: what it leaves to the L1 serves the edge lists)
   __shared__ __align__(16) int s_c1[BS_COLS / 8][12];  // per sector and column: cutoff + 1
@@ -349,12 +445,13 @@ __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G) {
     s_c1[c >> 3][c & 7u] = c < Gp ? (int)(min(b->cutc[c], 0x7FFFFFFEu) + 1u) : 0;
   __syncthreads();
   // hop-bounded round r: sources in table r (the members at 0 for r = 0), targets in
-  // table r + 1; a round's paths extend only while they have fewer than D edges
+  // table r + 1; a round announces only to a next one that pushes
   const uint32_t D = b->D, r = b->round, cls = b->cls, chunk_edges = b->chunk, cap = b->item_cap;
   const bool over = (D && r >= D) || b->error;  // past the last round: nothing to relax
+  const uint32_t pushes = D ? b->pull : 0u;     // the rounds that announce for a next one
   const uint32_t* src_tab = D ? (r ? b->tab[min(r, D)] : nullptr) : b->dist;
   uint32_t* dst_tab = D ? b->tab[min(r + 1u, D)] : b->dist;
-  const bool extend = D == 0u || r + 1u < D;
+  const bool extend = D == 0u || r + 1u < pushes;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
   // neighbouring takes go to different blocks: the first ones hold the hubs' chunks
@@ -404,8 +501,8 @@ __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G) {
       const uint32_t chunk = __shfl_sync(0xffffffffu, item.y, (int)own);
       const uint32_t m = (__ldcg(&b->am[(uint64_t)v * Wm + (sec >> 2)]) >> ((sec & 3u) * 8u)) & 0xFFu;
       uint4 da = make_uint4(0, 0, 0, 0), db = da;  // round 0: the members themselves
-      if (src_tab) {
-        const uint4* src = (const uint4*)&src_tab[(uint64_t)v * Gp + sec * 8];
+      if (PULL || src_tab) {
+        const uint4* src = (const uint4*)&(PULL ? dst_tab : src_tab)[(uint64_t)v * Gp + sec * 8];
         da = __ldcg(src);
         db = __ldcg(src + 1);
       }
@@ -418,11 +515,17 @@ __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G) {
 #pragma unroll
       for (int i = 0; i < 8; i++) {
         const int c1 = s_c1[sec][i];
-        const bool on = ((m >> i) & 1u) && dv[i] < (uint32_t)c1 - 1u;
-        x.nd[i] = on ? -(int)dv[i] : -0x7FFFFFFF;
-        wl = max(wl, c1 + x.nd[i] - 1);
+        if (PULL) {
+          x.nd[i] = (int)min(dv[i], (uint32_t)c1);
+          wl = max(wl, x.nd[i] - 1);
+        } else {
+          const bool on = ((m >> i) & 1u) && dv[i] < (uint32_t)c1 - 1u;
+          x.nd[i] = on ? -(int)dv[i] : -0x7FFFFFFF;
+          wl = max(wl, c1 + x.nd[i] - 1);
+        }
       }
       x.sec = sec;
+      x.at = v * nsec + sec;
       s_unit[wib][lane] = x;
       // the units of one item are neighbours: `lead` its first lane in the window, `cnt`
       // their number; the item's edges up to the largest limit among them
@@ -489,36 +592,52 @@ __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G) {
           at[y] = tu[y] * nsec + s_unit[wib][un[y]].sec;
           ra[y] = rb[y] = make_uint4(0, 0, 0, 0);
           if (ok[y]) {
-            ra[y] = __ldcg((const uint4*)(dst_tab + (uint64_t)at[y] * 8u));
-            rb[y] = __ldcg((const uint4*)(dst_tab + (uint64_t)at[y] * 8u) + 1);
+            const uint4* row = (const uint4*)((PULL ? src_tab : dst_tab) + (uint64_t)at[y] * 8u);
+            ra[y] = __ldcg(row);
+            rb[y] = __ldcg(row + 1);
           }
         }
 #pragma unroll
         for (int y = 0; y < BS_U; y++) {
           if (!ok[y]) continue;
           const BsUnit& q = s_unit[wib][un[y]];
-          const int* c1 = s_c1[q.sec];
+          [[maybe_unused]] const int* c1 = s_c1[q.sec];
           const int w = tw[y];
           const uint32_t du[8] = {ra[y].x, ra[y].y, ra[y].z, ra[y].w, rb[y].x, rb[y].y, rb[y].z, rb[y].w};
           int best = -0x7FFFFFFF;
+          if constexpr (PULL) {
+            BsUnit& t = s_unit[wib][un[y]];
 #pragma unroll
-          for (int i = 0; i < 8; i++)
-            best = __viaddmax_s32((int)min(du[i], (uint32_t)c1[i]), q.nd[i], best);
-          if (best <= w) continue;
-          uint32_t imp = 0, ann = 0;
+            for (int i = 0; i < 8; i++) best = max(best, t.nd[i] - (int)min(du[i], 0x7FFFFFFFu));
+            if (best <= w) continue;
 #pragma unroll
-          for (int i = 0; i < 8; i++)
-            imp |= (int)min(du[i], (uint32_t)c1[i]) + q.nd[i] > w ? 1u << i : 0u;
-          for (; imp; imp &= imp - 1u) {
-            const int i = __ffs(imp) - 1;
-            const int nd = w - q.nd[i];
-            atomicMin(dst_tab + (uint64_t)at[y] * 8u + i, (uint32_t)nd);
-            if (extend && nd + 1 < c1[i]) ann |= 1u << i;
-          }
-          if (ann) {
-            const uint32_t col = q.sec * 8u;
-            atomicOr(&fo[(uint64_t)tu[y] * Wm + (col >> 5)], ann << (col & 31u));
-            any = 1u;
+            for (int i = 0; i < 8; i++) {
+              const uint32_t nd = du[i] + (uint32_t)w;
+              if (du[i] < 0x7F000000u && nd < (uint32_t)t.nd[i]) {
+                atomicMin(&t.nd[i], (int)nd);
+                atomicMin(dst_tab + (uint64_t)t.at * 8u + i, nd);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+              best = __viaddmax_s32((int)min(du[i], (uint32_t)c1[i]), q.nd[i], best);
+            if (best <= w) continue;
+            uint32_t imp = 0, ann = 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+              imp |= (int)min(du[i], (uint32_t)c1[i]) + q.nd[i] > w ? 1u << i : 0u;
+            for (; imp; imp &= imp - 1u) {
+              const int i = __ffs(imp) - 1;
+              const int nd = w - q.nd[i];
+              atomicMin(dst_tab + (uint64_t)at[y] * 8u + i, (uint32_t)nd);
+              if (extend && nd + 1 < c1[i]) ann |= 1u << i;
+            }
+            if (ann) {
+              const uint32_t col = q.sec * 8u;
+              atomicOr(&fo[(uint64_t)tu[y] * Wm + (col >> 5)], ann << (col & 31u));
+              any = 1u;
+            }
           }
         }
       }
@@ -535,28 +654,14 @@ __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G) {
 }
 
 // Hop-bounded tables (n4 = V x Gp / 4 uint4 per table).  Before round r >= 1:
-// table r + 1 := table r.  With `finish`, after the search: every table above the last
-// round's target := that target (the search ended early; no path has more edges).
-__global__ void k_bs_copy(BsCtx* b, int64_t n4, int finish) {
-  const uint32_t D = b->D;
-  if (!D) return;
-  uint32_t from, h1;  // tables from + 1..h1 := table from
-  if (!finish) {
-    if (b->done || b->round == 0u || b->round >= D) return;
-    from = b->round;
-    h1 = from + 1u;
-  } else {
-    if (b->error) return;
-    from = b->round + 1u;
-    h1 = D;
-  }
-  if (from >= h1) return;
-  const uint4* src = (const uint4*)b->tab[from];
+// table r + 1 := table r.
+__global__ void k_bs_copy(BsCtx* b, int64_t n4) {
+  if (b->done || b->round == 0u || b->round >= b->D) return;
+  const uint4* src = (const uint4*)b->tab[b->round];
+  uint4* dst = (uint4*)b->tab[b->round + 1u];
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const uint4 x = __ldcs(src + i);
-    for (uint32_t h = from + 1u; h <= h1; h++) __stcs((uint4*)b->tab[h] + i, x);
-  }
+       i += (int64_t)gridDim.x * blockDim.x)
+    __stcs(dst + i, __ldcs(src + i));
 }
 
 }  // namespace gst

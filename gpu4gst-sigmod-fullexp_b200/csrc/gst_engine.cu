@@ -883,6 +883,7 @@ struct Runner {
     const size_t o_am = take(words);
     const int ncls = D ? 1 : search_classes(ncols);
     const size_t o_later = take(ncls > 1 ? words : 0);
+    const size_t o_near0 = take(D > 1 ? words : 0), o_near1 = take(D > 3 ? words : 0);
     const size_t o_items = take((size_t)item_cap * 8);
     const size_t o_cols = take((size_t)BS_COLS * 4);
     void* p = nullptr;
@@ -907,6 +908,11 @@ struct Runner {
     h.ncls = (uint32_t)ncls;
     h.later = ncls > 1 ? (uint32_t*)(base + o_later) : nullptr;
     h.cend = g->d_cend;
+    // the rounds that pull: the last one from D = 2 on, the one before it from D = 4 on (at
+    // D = 3 the vertices it would pull at are those it pushes from)
+    h.pull = D > 3 ? D - 2 : D > 1 ? D - 1 : D;
+    h.near[0] = D > 1 ? (uint32_t*)(base + o_near0) : nullptr;
+    h.near[1] = D > 3 ? (uint32_t*)(base + o_near1) : nullptr;
     h.items = (uint2*)(base + o_items);
     h.item_cap = (uint32_t)item_cap;
     h.chunk = chunk;
@@ -926,6 +932,11 @@ struct Runner {
         h.qcol[q][i] =
             (uint16_t)(std::find(cols.begin(), cols.end(), jobs[q]->gids[i]) - cols.begin());
     }
+    for (size_t q = 0; q < jobs.size(); q++) {
+      uint32_t sectors = 0;
+      for (int i = 0; i < jobs[q]->q.k; i++) sectors |= 1u << (h.qcol[q][i] / 8);
+      for (int i = 0; i < jobs[q]->q.k; i++) h.colsec[h.qcol[q][i]] |= sectors;
+    }
     for (int c = 0; c < BS_COLS; c++) h.cutc[c] = COST_INF;
     cudaStream_t st = eng->stream;
     BsCtx* d_b = (BsCtx*)(base + o_b);
@@ -940,6 +951,8 @@ struct Runner {
     CK(cudaMemsetAsync(h.fm[0], 0, words, st));
     CK(cudaMemsetAsync(h.fm[1], 0, words, st));
     if (ncls > 1) CK(cudaMemsetAsync(h.later, 0, words, st));
+    for (uint32_t* near : h.near)
+      if (near) CK(cudaMemsetAsync(near, 0, words, st));
     CK(cudaMemcpyAsync(d_b, &h, sizeof(BsCtx), cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_cols, cols.data(), ncols * 4, cudaMemcpyHostToDevice, st));
     cs.h2d += sizeof(BsCtx) + ncols * 4;
@@ -948,21 +961,25 @@ struct Runner {
     int64_t launches = 1, relax_launches = 0;
     const int64_t n4 = V * (int64_t)Gp / 4;
     int occ = 1;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bs_relax, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bs_relax<false>, 256, 0);
     const int relax_blocks = eng->sms * std::max(1, std::min(occ, 4));
     const bool wide = V >= 600000;  // four vertices per scan thread
     const int scan_blocks = (int)std::min<int64_t>(eng->sms * 8, wide ? (V + 1023) / 1024 : (V + 255) / 256);
     BsCtx hb;
     for (;;) {
-      for (int i = 0; i < 6; i++) {
-        if (D) {
-          k_bs_copy<<<eng->sms * 4, 256, 0, st>>>(d_b, n4, 0);
+      // a hop-bounded search has D steps; an unbounded one is looked at every six
+      for (int i = 0; i < (D ? D : 6); i++) {
+        if (D && i) {
+          k_bs_copy<<<eng->sms * 4, 256, 0, st>>>(d_b, n4);
           launches++;
         }
-        if (wide) k_bs_scan<4><<<scan_blocks, 256, 0, st>>>(d_b, G);
-        else k_bs_scan<1><<<scan_blocks, 256, 0, st>>>(d_b, G);
+        const bool pull = D && (uint32_t)i >= h.pull;
+        auto* scan = wide ? (pull ? k_bs_scan<4, true> : k_bs_scan<4, false>)
+                          : (pull ? k_bs_scan<1, true> : k_bs_scan<1, false>);
+        scan<<<scan_blocks, 256, 0, st>>>(d_b, G);
         const int pe = prof_begin(PROF_BSRELAX);
-        k_bs_relax<<<relax_blocks, 256, 0, st>>>(d_b, G);
+        if (pull) k_bs_relax<true><<<relax_blocks, 256, 0, st>>>(d_b, G);
+        else k_bs_relax<false><<<relax_blocks, 256, 0, st>>>(d_b, G);
         prof_end(pe);
         relax_launches++;
         launches += 2;
@@ -971,12 +988,7 @@ struct Runner {
       CK(cudaMemcpyAsync(&hb, d_b, sizeof(BsCtx), cudaMemcpyDeviceToHost, st));
       cs.d2h += sizeof(BsCtx);
       CK(cudaStreamSynchronize(st));
-      if (hb.done) break;
-    }
-    if (D && hb.round + 1u < (uint32_t)D) {
-      k_bs_copy<<<eng->sms * 4, 256, 0, st>>>(d_b, n4, 1);
-      launches++;
-      CK(cudaGetLastError());
+      if (hb.done || D) break;
     }
     CK(cudaEventRecord(eng->bs_ev[1], st));
     CK(cudaEventSynchronize(eng->bs_ev[1]));
