@@ -624,27 +624,79 @@ __device__ __forceinline__ void add_stat(Ctx* ctxs, int qi, bool valid, uint32_t
 }
 
 // ---- admission: the per-vertex buffers of queries that start together -----------------
-// One pass over the vertices for all of them: empty row maps, dirty bits and frontier
-// bytes, the state rows the slot's last query wrote, and the distance rows, gathered from
-// a shared search's tables or the group cache (or left unreached for the query's own
-// search).  Gathered distances are final, so the same pass takes what the bounds need of
-// them: the star bound min_v sum_i d_i(v) (the cost of the k shortest paths from the best
-// centre v, a feasible tree, so a valid ub), for a hop-bounded query also the best star of
-// D/2-edge paths (see k_sssp), and the group distances vv.  The queries of a batch read the
-// rows of one shared table, so a block takes them through its vertices one after another:
-// the row is read from memory once.  With up to twelve fills, gathers and passes per query
-// instead, starting 100 queries over 20k vertices took 3.5 ms more (call 12.7 to 10.2 ms),
-// 32 hop-bounded ones over 1M vertices 3 ms (32 to 28.7 ms).
+// k_admit, one pass over the vertices for all of them: empty row maps, dirty bits and
+// frontier bytes, the state rows the slot's last query wrote, and for queries that do not
+// come from a shared search the distance rows, from the group cache or unreached.  With up
+// to twelve fills, gathers and passes per query instead, starting 100 queries over 20k
+// vertices took 3.5 ms more (call 12.7 to 10.2 ms).
+// k_gather, the distance rows of queries that come from shared searches: a block loads
+// whole rows of a shared table into shared memory, one span, and writes every query's
+// columns of them from there.  Each lane reading its own columns from the table, in the
+// pass of k_admit, took 10.7 ms for the 4M-vertex batch; now 4.5 ms, and 0.8 of k_admit (16 GB
+// in all: 3.6 TB/s).
 struct AdmitQ {
   uint32_t slot;
-  uint32_t gather;                       // distances come from src; the bounds follow
-  uint32_t stride;                       // uint32 between a source's vertices
-  uint32_t pad;
-  uint64_t dirty16;                      // 16-byte words of the table to clear
+  uint32_t rows;     // distance rows: 0 unreached, 1 from src, 2 by k_gather
+  uint64_t dirty16;  // 16-byte words of the table to clear
   // src[h][i]: group i's distances to every vertex within hop budget h (h = 0: the distance
   // table itself); nullptr: unreached
   const uint32_t* src[HOP_BUDGETS_MAX + 1][KMAX];
 };
+struct GatherSrc {   // a table of a shared search
+  const uint32_t* tab;
+  uint32_t Gp;       // its columns
+  uint32_t first, n; // its entries
+};
+struct GatherEnt {   // columns of it that are a query's distances within budget h
+  uint16_t slot, h;
+  uint16_t col[KMAX];
+};
+constexpr int GATHER_V = 64;  // vertices per block and tile of k_gather
+
+// Store vertex v's distances d within budget h of a starting query.  The distances of a
+// query in PH_PREP are final, so what the bounds need of them is taken here: *best, the star
+// bound min_v sum_i d_i(v) (the cost of the k shortest paths from the best centre v, a
+// feasible tree, so a valid ub), for a hop-bounded query *best_h, the best star of D/2-edge
+// paths (see k_sssp), and the group distances vv.
+__device__ __forceinline__ void admit_row(Ctx* c, int64_t V, int64_t v, int h, const uint32_t d[KMAX],
+                                          uint32_t* best, uint32_t* best_h) {
+  const int k = c->k;
+  const uint32_t ds = c->ds;
+  store_drow(h ? c->dist_h + (uint64_t)(h - 1) * (uint64_t)V * ds : c->dist, ds, (uint64_t)v,
+             make_uint4(d[0], d[1], d[2], d[3]), make_uint4(d[4], d[5], d[6], d[7]));
+  if (c->phase != PH_PREP) return;
+  const int hs = c->hop && c->sssp_hops && c->D / 2 <= c->nhb ? c->D / 2 : -1;
+  uint64_t sum = 0;
+#pragma unroll
+  for (int i = 0; i < KMAX; i++) sum += i < k ? d[i] : 0u;
+  if (h == hs && h > 0) *best_h = (uint32_t)min(sum, (uint64_t)COST_INF);
+  if (h != 0) return;
+  *best = (uint32_t)min(sum, (uint64_t)COST_INF);
+  bool all = true, some = false;
+#pragma unroll
+  for (int i = 0; i < KMAX; i++) {
+    all = all && (i >= k || d[i] == 0u);
+    some = some || (i < k && d[i] == 0u);
+  }
+  if (hs == 0 && all) *best_h = 0u;  // budget 0: the members themselves
+  if (some)
+#pragma unroll
+    for (int i = 0; i < KMAX; i++)
+      if (i < k && d[i] == 0u) {
+#pragma unroll
+        for (int j = 0; j < KMAX; j++)
+          if (j < k && d[j] < __ldcg(&c->vv[i * KMAX + j])) atomicMin(&c->vv[i * KMAX + j], d[j]);
+      }
+}
+// A block's best stars of a query into its bounds.
+__device__ __forceinline__ void admit_bounds(Ctx* c, uint32_t best, uint32_t best_h) {
+  if (c->phase != PH_PREP) return;
+  if (best < COST_INF) atomicMin(&c->ub, best);
+  // ub_cell bounds with strict tests (a state must beat a tree already found), so a
+  // feasible cost that no state holds yet enters it plus one
+  if (best_h < COST_INF - 1u) atomicMin(&c->ub_cell, best_h + 1u);
+}
+
 __global__ void __launch_bounds__(256) k_admit(Ctx* ctxs, const AdmitQ* aq, int n, DevGraph G) {
   __shared__ uint32_t s_best[MAXB], s_hop[MAXB];
   for (int q = threadIdx.x; q < MAXB; q += blockDim.x) s_best[q] = s_hop[q] = COST_INF;
@@ -656,44 +708,19 @@ __global__ void __launch_bounds__(256) k_admit(Ctx* ctxs, const AdmitQ* aq, int 
     for (int q = 0; q < n; q++) {
       const AdmitQ& a = aq[q];
       Ctx* c = ctxs + a.slot;
-      const int k = c->k, nhb = c->nhb;
-      const uint32_t ds = c->ds;
       uint32_t best = COST_INF, best_h = COST_INF;
       if (live) {
         if (c->rowmap) c->rowmap[v] = ROW_NONE;
         if ((v & 31) == 0) c->rowbits[v >> 5] = 0u;
-        if (!a.gather || c->phase == PH_SSSP) {
-          if ((v & 3) == 0) c->fm[0][v >> 2] = c->fm[1][v >> 2] = 0u;
-        }
-        const int hs = c->hop && c->sssp_hops && c->D / 2 <= nhb ? c->D / 2 : -1;
-        for (int h = nhb; h >= 0; h--) {
+        if (c->phase == PH_SSSP && (v & 3) == 0) c->fm[0][v >> 2] = c->fm[1][v >> 2] = 0u;
+        for (int h = a.rows == 2u ? -1 : c->nhb; h >= 0; h--) {
           uint32_t d[KMAX];
-          uint64_t sum = 0;
 #pragma unroll
           for (int i = 0; i < KMAX; i++) {
-            const uint32_t* src = i < k && a.gather ? a.src[h][i] : nullptr;
-            d[i] = src ? src[v * (int64_t)a.stride] : COST_INF;
-            sum += i < k ? d[i] : 0u;
+            const uint32_t* src = i < c->k && a.rows ? a.src[h][i] : nullptr;
+            d[i] = src ? src[v] : COST_INF;
           }
-          store_drow(h ? c->dist_h + (uint64_t)(h - 1) * (uint64_t)G.V * ds : c->dist, ds, (uint64_t)v,
-                     make_uint4(d[0], d[1], d[2], d[3]), make_uint4(d[4], d[5], d[6], d[7]));
-          if (h && h == hs) best_h = (uint32_t)min(sum, (uint64_t)COST_INF);
-          if (h == 0 && c->phase == PH_PREP) {
-            best = (uint32_t)min(sum, (uint64_t)COST_INF);
-            if (hs == 0) {  // budget 0: the members themselves
-              bool all = true;
-#pragma unroll
-              for (int i = 0; i < KMAX; i++) all = all && (i >= k || d[i] == 0u);
-              best_h = all ? 0u : COST_INF;
-            }
-#pragma unroll
-            for (int i = 0; i < KMAX; i++)
-              if (i < k && d[i] == 0u) {
-#pragma unroll
-                for (int j = 0; j < KMAX; j++)
-                  if (j < k && d[j] < __ldcg(&c->vv[i * KMAX + j])) atomicMin(&c->vv[i * KMAX + j], d[j]);
-              }
-          }
+          admit_row(c, G.V, v, h, d, &best, &best_h);
         }
       }
       best = __reduce_min_sync(0xffffffffu, best);
@@ -711,14 +738,54 @@ __global__ void __launch_bounds__(256) k_admit(Ctx* ctxs, const AdmitQ* aq, int 
       t[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
   }
   __syncthreads();
-  for (int q = threadIdx.x; q < n; q += blockDim.x) {
-    Ctx* c = ctxs + aq[q].slot;
-    if (c->phase != PH_PREP) continue;
-    if (s_best[q] < COST_INF) atomicMin(&c->ub, s_best[q]);
-    // ub_cell bounds with strict tests (a state must beat a tree already found), so a
-    // feasible cost that no state holds yet enters it plus one
-    if (s_hop[q] < COST_INF - 1u) atomicMin(&c->ub_cell, s_hop[q] + 1u);
+  for (int q = threadIdx.x; q < n; q += blockDim.x) admit_bounds(ctxs + aq[q].slot, s_best[q], s_hop[q]);
+}
+
+// Dynamic shared memory: GATHER_V rows of the widest table, a word more per row (the columns
+// of neighbouring vertices then lie in different banks).
+__global__ void __launch_bounds__(256) k_gather(Ctx* ctxs, const GatherSrc* srcs, const GatherEnt* ents,
+                                             DevGraph G) {
+  extern __shared__ uint32_t s_tile[];
+  __shared__ uint32_t s_best[MAXB], s_hop[MAXB];
+  const GatherSrc s = srcs[blockIdx.y];
+  const uint32_t Gp = s.Gp, Gq = Gp / 4u, pitch = Gp + 1u;
+  for (int q = threadIdx.x; q < MAXB; q += blockDim.x) s_best[q] = s_hop[q] = COST_INF;
+  for (int64_t v0 = (int64_t)blockIdx.x * GATHER_V; v0 < G.V; v0 += (int64_t)gridDim.x * GATHER_V) {
+    const uint32_t nv = (uint32_t)min((int64_t)GATHER_V, G.V - v0);
+    const uint4* rows = (const uint4*)(s.tab + v0 * Gp);
+    __syncthreads();  // the tile is free
+    for (uint32_t i = threadIdx.x; i < nv * Gq; i += blockDim.x) {
+      const uint4 x = __ldcs(rows + i);
+      const uint32_t v = i / Gq;
+      uint32_t* t = s_tile + v * pitch + (i - v * Gq) * 4u;
+      t[0] = x.x;
+      t[1] = x.y;
+      t[2] = x.z;
+      t[3] = x.w;
+    }
+    __syncthreads();
+    for (uint32_t p = threadIdx.x; p < s.n * GATHER_V; p += blockDim.x) {
+      const uint32_t v = p % GATHER_V, q = p / GATHER_V;  // a warp: one entry
+      const GatherEnt& e = ents[s.first + q];
+      Ctx* c = ctxs + e.slot;
+      uint32_t best = COST_INF, best_h = COST_INF;
+      if (v < nv) {
+        uint32_t d[KMAX];
+#pragma unroll
+        for (int i = 0; i < KMAX; i++) d[i] = i < c->k ? s_tile[v * pitch + e.col[i]] : COST_INF;
+        admit_row(c, G.V, v0 + v, e.h, d, &best, &best_h);
+      }
+      best = __reduce_min_sync(0xffffffffu, best);
+      best_h = __reduce_min_sync(0xffffffffu, best_h);
+      if ((threadIdx.x & 31) == 0) {
+        if (best < s_best[q]) atomicMin(&s_best[q], best);
+        if (best_h < s_hop[q]) atomicMin(&s_hop[q], best_h);
+      }
+    }
   }
+  __syncthreads();
+  for (uint32_t q = threadIdx.x; q < s.n; q += blockDim.x)
+    admit_bounds(ctxs + ents[s.first + q].slot, s_best[q], s_hop[q]);
 }
 
 // ---- init: group members -> zero-cost singletons, SSSP sources, dirty rows ----

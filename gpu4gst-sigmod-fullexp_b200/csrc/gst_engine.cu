@@ -432,6 +432,13 @@ struct Runner {
   AdmitQ* d_aq = nullptr;       // MAXB: the queries start_admitted() starts
   AdmitQ* h_aq = nullptr;       // pinned: those admitted since its last call
   int n_aq = 0;
+  // their columns of shared tables, by table and width; the same as two arrays on the device
+  std::map<std::pair<const uint32_t*, uint32_t>, std::vector<GatherEnt>> gathers;
+  static constexpr int kGathers = MAXB * (HOP_BUDGETS_MAX + 1);
+  GatherSrc* d_gsrc = nullptr;
+  GatherEnt* d_gent = nullptr;
+  GatherSrc* h_gsrc = nullptr;  // pinned
+  GatherEnt* h_gent = nullptr;  // pinned
   LoopCtl* d_loop = nullptr;    // counters of the level loop
   uint32_t* loop_init = nullptr;  // pinned: values for d_loop before a launch
   uint32_t* loop_left = nullptr;  // pinned: iterations left after it
@@ -494,6 +501,12 @@ struct Runner {
     if (d_aq) cudaFree(d_aq);
     if (h_aq) cudaFreeHost(h_aq);
     d_aq = h_aq = nullptr;
+    if (d_gsrc) cudaFree(d_gsrc);
+    if (d_gent) cudaFree(d_gent);
+    if (h_gsrc) cudaFreeHost(h_gsrc);
+    if (h_gent) cudaFreeHost(h_gent);
+    d_gsrc = h_gsrc = nullptr;
+    d_gent = h_gent = nullptr;
     if (d_loop) cudaFree(d_loop);
     if (loop_init) cudaFreeHost(loop_init);
     loop_init = loop_left = nullptr;
@@ -507,6 +520,10 @@ struct Runner {
     CK(cudaMallocHost(&h_ctx, sizeof(Ctx) * MAXB));
     CK(cudaMalloc(&d_aq, sizeof(AdmitQ) * MAXB));
     CK(cudaMallocHost(&h_aq, sizeof(AdmitQ) * MAXB));
+    CK(cudaMalloc(&d_gsrc, sizeof(GatherSrc) * kGathers));
+    CK(cudaMalloc(&d_gent, sizeof(GatherEnt) * kGathers));
+    CK(cudaMallocHost(&h_gsrc, sizeof(GatherSrc) * kGathers));
+    CK(cudaMallocHost(&h_gent, sizeof(GatherEnt) * kGathers));
     CK(cudaMalloc(&d_loop, sizeof(LoopCtl)));
     CK(cudaMemset(d_loop, 0, sizeof(LoopCtl)));
     CK(cudaMallocHost(&loop_init, sizeof(uint32_t) * 4));
@@ -745,7 +762,6 @@ struct Runner {
     AdmitQ& a = h_aq[n_aq];
     memset(&a, 0, sizeof(a));
     a.slot = (uint32_t)s;
-    a.stride = 1;
     int n_cached = 0;
     const size_t V = (size_t)g->V;
     if (!hop && !j->cache_dst) {
@@ -763,12 +779,16 @@ struct Runner {
     Shared* S = shared_of(*j);
     if (S) {
       c.cut_fix = std::max(1u, j->ss_cut);
-      a.stride = S->Gp;
-      for (int h = 0; h <= c.nhb; h++)
-        for (int i = 0; i < q->k; i++) a.src[h][i] = (h ? S->tab[h] : S->dist) + j->ss_cols[i];
+      for (int h = 0; h <= c.nhb; h++) {
+        GatherEnt ent{};
+        ent.slot = (uint16_t)s;
+        ent.h = (uint16_t)h;
+        for (int i = 0; i < q->k; i++) ent.col[i] = j->ss_cols[i];
+        gathers[{h ? S->tab[h] : S->dist, S->Gp}].push_back(ent);
+      }
       S->remaining--;
     }
-    a.gather = n_cached > 0 || S;
+    a.rows = S ? 2u : n_cached > 0 ? 1u : 0u;
     if (S || n_cached == q->k) c.phase = PH_PREP;
     if (!S && n_cached == q->k) c.sssp_full = 1;
     c.sssp_mask = c.sssp_hops ? 2u : (c.bucket_end == 0xFFFFFFFFu ? 1u : 0u);
@@ -816,6 +836,22 @@ struct Runner {
     cs.h2d += (int64_t)(sizeof(Ctx) + sizeof(AdmitQ)) * n;
     const int blocks = (int)std::min<int64_t>(eng->sms * 8, (g->V + 255) / 256);
     k_admit<<<blocks, 256, 0, st>>>(d_ctx, d_aq, n, G);
+    if (!gathers.empty()) {
+      int ns = 0, ne = 0;
+      uint32_t widest = 0;
+      for (const auto& x : gathers) {
+        h_gsrc[ns++] = GatherSrc{x.first.first, x.first.second, (uint32_t)ne, (uint32_t)x.second.size()};
+        for (const GatherEnt& ent : x.second) h_gent[ne++] = ent;
+        widest = std::max(widest, x.first.second);
+      }
+      gathers.clear();
+      CK(cudaMemcpyAsync(d_gsrc, h_gsrc, sizeof(GatherSrc) * ns, cudaMemcpyHostToDevice, st));
+      CK(cudaMemcpyAsync(d_gent, h_gent, sizeof(GatherEnt) * ne, cudaMemcpyHostToDevice, st));
+      cs.h2d += (int64_t)(sizeof(GatherSrc) * ns + sizeof(GatherEnt) * ne);
+      const int tiles = (int)std::min<int64_t>(eng->sms * 8, (g->V + GATHER_V - 1) / GATHER_V);
+      k_gather<<<dim3(tiles, ns), 256, GATHER_V * (widest + 1) * 4, st>>>(d_ctx, d_gsrc, d_gent, G);
+      cs.launches += 1;
+    }
     k_init<<<dim3(8, n, KMAX), 256, 0, st>>>(d_ctx, d_aq, n, G, grp->d_ptr, grp->d_mem);
     const int tour_bytes = (1 << kmax) * TOUR_STRIDE * 4;
     k_ctrl<<<n, 512, tour_bytes, st>>>(d_ctx, d_aq, n, tour_bytes);
@@ -1551,7 +1587,9 @@ gst_status gst_engine_create(int32_t device, const gst_config* cfg, gst_engine**
   if (cudaFuncSetAttribute(k_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)eng->rows_smem) != cudaSuccess ||
       cudaFuncSetAttribute(k_ctrl, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (1 << KMAX) * TOUR_STRIDE * 4) != cudaSuccess) {
+                           (1 << KMAX) * TOUR_STRIDE * 4) != cudaSuccess ||
+      cudaFuncSetAttribute(k_gather, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           GATHER_V * (BS_COLS + 1) * 4) != cudaSuccess) {
     cudaStreamDestroy(eng->stream);
     cudaMemPoolDestroy(eng->pool);
     delete eng;
