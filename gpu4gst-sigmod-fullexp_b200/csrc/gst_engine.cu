@@ -76,7 +76,8 @@ constexpr uint32_t kStackCap = 1u << 18;
 
 constexpr size_t kDenseBytes = (size_t)32 << 20;  // tables laid out densely up to here,
 constexpr int64_t kDenseVertices = 1 << 17;       // or to here
-constexpr size_t kPoolRoom = (size_t)2 << 30;     // bytes a row pool may take beyond its eighth
+constexpr size_t kPoolBytes = (size_t)256 << 20;  // bytes of rows worth having in any case,
+constexpr size_t kPoolRoom = (size_t)3 << 29;     // and at most beyond an eighth of the vertices
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -91,15 +92,18 @@ bool dense_rows(int64_t V, size_t rw, uint64_t rows, int boost) {
   return rows >= (uint64_t)V &&
          ((size_t)V * rw * 8 <= kDenseBytes || V <= kDenseVertices || boost > 0);
 }
-// Rows of a query's row pool: an eighth of the vertices (at least 64k rows), or as many as
-// `room` bytes hold, four times more per capacity retry; at most 5/4 of the vertices, since
-// every lost race for a row leaves one unused, or one per vertex in the dense layout.  Most
-// queries write rows for a few percent of the vertices (their pruning keeps the DP near the
-// optimal trees), but the heaviest k = 7 ones overflow an eighth and then run twice, the
-// second time with a search of their own (10 to 22 of 155 ms of a batch of 32 over 4M
-// vertices, the lost first run not counted: 129 ms without).
+// Rows of a query's row pool: an eighth of the vertices (at least 64k rows); where `room`
+// bytes hold more, three eighths of them or 256 MB of rows; four times more per capacity
+// retry; at most 5/4 of the vertices, since every lost race for a row leaves one unused, or
+// one per vertex in the dense layout.  Most queries write rows for a few percent of the
+// vertices (their pruning keeps the DP near the optimal trees), but the heaviest k = 7 ones
+// overflow an eighth and then run twice, the second time with a search of their own (10 to
+// 22 of 155 ms of a batch of 32 over 4M vertices, the lost first run not counted: 129 ms
+// without).  No more than that: fresh memory costs its mapping and one clearing.
 uint32_t pool_rows(int64_t V, size_t rw, size_t room, int boost) {
-  uint64_t r = std::max<uint64_t>(std::max<uint64_t>(1u << 16, (uint64_t)V / 8), room / (rw * 8));
+  const uint64_t more = std::max<uint64_t>((uint64_t)V / 8 * 3, kPoolBytes / (rw * 8));
+  uint64_t r = std::max<uint64_t>(1u << 16, (uint64_t)V / 8);
+  r = std::max<uint64_t>(r, std::min<uint64_t>(more, room / (rw * 8)));
   for (int i = 0; i < boost; i++) r = std::min<uint64_t>(r * 4, 1u << 30);
   if (dense_rows(V, rw, r, boost)) return (uint32_t)V;
   return (uint32_t)std::min<uint64_t>(r, (uint64_t)V + (uint64_t)V / 4);
@@ -151,12 +155,14 @@ int hop_budgets(int D) { return D > 1 ? std::min(D - 1, HOP_BUDGETS_MAX) : 0; }
 
 // Worklist capacity.  A level appends at most one item per edge chunk of every
 // state it settles, which in the worst case is every cell of the slab; queries
-// use a small fraction of that, so a slot starts at `base` items and a query that
-// overflows is re-run with four times the room (up to the worst case).
+// use a small fraction of that, so a slot starts at 8 items per vertex, from 1M vertices on
+// 4 (the heaviest k = 7 queries over 4M vertices fill 1.04), and a query that overflows is
+// re-run with four times the room (up to the worst case).
 uint32_t list_cap(int64_t V, int64_t E, size_t rw, int split, int boost) {
   const uint64_t worst = std::min<uint64_t>((uint64_t)V * rw + (uint64_t)E / split * rw + 4096,
                                             (1ull << 31));
-  uint64_t c = std::max<uint64_t>(1ull << 16, 8ull * (uint64_t)V + 2ull * (uint64_t)E / split);
+  const uint64_t per = std::max<uint64_t>(std::min<uint64_t>(8ull * (uint64_t)V, 8ull << 20), 4ull * (uint64_t)V);
+  uint64_t c = std::max<uint64_t>(1ull << 16, per + 2ull * (uint64_t)E / split);
   for (int i = 0; i < boost; i++) c *= 4;
   return (uint32_t)std::min(c, worst);
 }
