@@ -112,7 +112,7 @@ constexpr uint32_t ROW_NONE = 0xFFFFFFFFu;
 constexpr int WIDX = 16;
 constexpr uint32_t CHUNK = 0x80000000u;  // item flag (in pd): one `split`-edge chunk only
 constexpr uint32_t GROW_TAKE = 16;       // grow items a warp takes at a time, at most
-constexpr int RELAX_U = 4;               // edges per lane per round of the grow relax loop
+constexpr int RELAX_U = 2;               // edges per lane per round of the grow relax loop
 // Hop-limited distance items carry their path's edge count in bits 8..15 of the
 // group word (group index in bits 0..7).
 constexpr uint32_t SSSP_HOP_SHIFT = 8;
@@ -1212,11 +1212,14 @@ __device__ __forceinline__ void ctrl_grow(Ctx* c) {
 // first take of a warp is its own share, the further ones come from a counter.  Three
 // hop-bounded queries over 1M vertices: grow 4.7 to 1.4 ms, three queries k = 5/7 over
 // 141k: 3.0 to 1.5 ms.  With 8 items at most the 141k batch takes 5.6 ms instead of 4.9,
-// with 32 the 1M batch 4.0 instead of 3.4.
+// with 32 the 1M batch 4.0 instead of 3.4.  An item relaxes 17 edges on average since the
+// rest bounds, so two edges per lane in flight and four blocks per SM (62 registers, no
+// spills) beat four and three (80, 168 bytes spilled): 4.8 to 4.3 ms on the 141k batch, 12.6
+// to 11.5 at 4M vertices; one edge per lane takes 4.4 and 11.6.
 // The last block runs the control step of every query; in the graph loop (in_loop) it
 // also decides whether the loop goes on: no resident query has finished,
 // some query is resident, iterations are left.
-__global__ void __launch_bounds__(256, 3) k_grow(Ctx* ctxs, int nctx, DevGraph G, int split, LoopCtl* lc,
+__global__ void __launch_bounds__(256, 4) k_grow(Ctx* ctxs, int nctx, DevGraph G, int split, LoopCtl* lc,
                                               cudaGraphConditionalHandle loop, int in_loop) {
   __shared__ uint32_t s_pref[MAXB + 1];
   load_prefix(ctxs, nctx, s_pref, PH_DP);
