@@ -432,8 +432,10 @@ struct __align__(16) BsWork {  // one item of a window with work
                                // pair's edge is (pair * that) >> 16, exact below 2^11 pairs
 };
 // PULL: the items are targets; a pair reads the neighbour's row and lowers the item's.
+// in_loop: the launch is the last node of a graph loop over the steps, which it ends.
 template <bool PULL>
-__global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G) {
+__global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G, cudaGraphConditionalHandle loop,
+                                                  int in_loop) {
   // (shared memory is kept small: what it leaves to the L1 serves the edge lists)
   __shared__ __align__(16) int s_c1[BS_COLS / 8][12];  // per sector and column: cutoff + 1
   __shared__ BsUnit s_unit[256 / 32][32];              // per warp: the window's units
@@ -650,7 +652,10 @@ __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G) {
   any = __reduce_or_sync(0xffffffffu, any);
   if (lane == 0 && any) b->ann = 1u;
   if (lane == 0 && relaxed) atomicAdd(&b->st_relax, relaxed);  // the same in every lane
-  if (last_block(&b->arrived) && threadIdx.x == 0) bs_advance(b);
+  if (last_block(&b->arrived) && threadIdx.x == 0) {
+    bs_advance(b);
+    if (in_loop) cudaGraphSetConditional(loop, b->done ? 0u : 1u);
+  }
 }
 
 // Hop-bounded tables (n4 = V x Gp / 4 uint4 per table).  Before round r >= 1:

@@ -435,6 +435,10 @@ struct Runner {
   std::vector<Arena> arenas;
   Ctx* d_ctx = nullptr;         // MAXB contexts
   Ctx* h_ctx = nullptr;         // pinned mirror
+  BsCtx* d_bs = nullptr;        // context of the shared search that runs
+  BsCtx* h_bs = nullptr;        // pinned
+  cudaGraph_t bs_graph = nullptr;  // the steps of an unbounded one
+  cudaGraphExec_t bs_exec = nullptr;
   AdmitQ* d_aq = nullptr;       // MAXB: the queries start_admitted() starts
   AdmitQ* h_aq = nullptr;       // pinned: those admitted since its last call
   int n_aq = 0;
@@ -469,7 +473,6 @@ struct Runner {
   struct Shared {
     void* mem = nullptr;
     size_t bytes = 0;
-    BsCtx* d_b = nullptr;
     int id = 0;
     int remaining = 0;               // its queries not admitted yet
     int D = 0;                       // 0: unbounded distances; else the hop bound
@@ -504,6 +507,13 @@ struct Runner {
     held = 0;
     if (d_ctx) cudaFree(d_ctx);
     if (h_ctx) cudaFreeHost(h_ctx);
+    if (bs_exec) cudaGraphExecDestroy(bs_exec);
+    if (bs_graph) cudaGraphDestroy(bs_graph);
+    bs_exec = nullptr;
+    bs_graph = nullptr;
+    if (d_bs) cudaFree(d_bs);
+    if (h_bs) cudaFreeHost(h_bs);
+    d_bs = h_bs = nullptr;
     if (d_aq) cudaFree(d_aq);
     if (h_aq) cudaFreeHost(h_aq);
     d_aq = h_aq = nullptr;
@@ -524,6 +534,8 @@ struct Runner {
   gst_status init() {
     CK(cudaMalloc(&d_ctx, sizeof(Ctx) * MAXB));
     CK(cudaMallocHost(&h_ctx, sizeof(Ctx) * MAXB));
+    CK(cudaMalloc(&d_bs, sizeof(BsCtx)));
+    CK(cudaMallocHost(&h_bs, sizeof(BsCtx)));
     CK(cudaMalloc(&d_aq, sizeof(AdmitQ) * MAXB));
     CK(cudaMallocHost(&h_aq, sizeof(AdmitQ) * MAXB));
     CK(cudaMalloc(&d_gsrc, sizeof(GatherSrc) * kGathers));
@@ -889,6 +901,41 @@ struct Runner {
     return pairs >= 5e8 || (sectors >= 12 && pairs >= 1.5e8) ? 2 : 1;
   }
 
+  // The steps of an unbounded shared search as a CUDA graph: a WHILE node whose body is one
+  // step (scan, relax), whose relax kernel decides whether to go on.
+  gst_status search_graph(bool wide, int scan_blocks, int relax_blocks, cudaGraphExec_t* out) {
+    if (!bs_exec) {
+      if (bs_graph) cudaGraphDestroy(bs_graph);
+      bs_graph = nullptr;
+      const DevGraph G = dev_graph(g);
+      CK(cudaGraphCreate(&bs_graph, 0));
+      cudaGraphConditionalHandle handle;
+      CK(cudaGraphConditionalHandleCreate(&handle, bs_graph, 1, cudaGraphCondAssignDefault));
+      cudaGraphNodeParams cp = {};
+      cp.type = cudaGraphNodeTypeConditional;
+      cp.conditional.handle = handle;
+      cp.conditional.type = cudaGraphCondTypeWhile;
+      cp.conditional.size = 1;
+      cudaGraphNode_t node;
+      CK(cudaGraphAddNode(&node, bs_graph, nullptr, 0, &cp));
+      cudaStream_t cap;
+      CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+      CK(cudaStreamBeginCaptureToGraph(cap, cp.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                       cudaStreamCaptureModeThreadLocal));
+      auto* scan = wide ? k_bs_scan<4, false> : k_bs_scan<1, false>;
+      scan<<<scan_blocks, 256, 0, cap>>>(d_bs, G);
+      k_bs_relax<false><<<relax_blocks, 256, 0, cap>>>(d_bs, G, handle, 1);
+      cudaGraph_t captured = nullptr;
+      const cudaError_t ce = cudaStreamEndCapture(cap, &captured);
+      cudaStreamDestroy(cap);
+      if (ce != cudaSuccess)
+        return fail(eng, GST_DEVICE_ERROR, std::string("graph capture: ") + cudaGetErrorString(ce));
+      CK(cudaGraphInstantiate(&bs_exec, bs_graph, 0));
+    }
+    *out = bs_exec;
+    return GST_OK;
+  }
+
   // One batch-shared distance search for the queries `jobs`, all unbounded (D = 0) or all
   // of hop bound D (1..KMAX), over their distinct groups `cols` (at most BS_COLS groups,
   // BS_MAXQ queries).  On success every job is marked (ss = 1) with its columns and
@@ -917,7 +964,6 @@ struct Runner {
       off = align256(off + n);
       return o;
     };
-    const size_t o_b = take(sizeof(BsCtx));
     const size_t o_dist = take((size_t)V * Gp * 4 * (size_t)std::max(D, 1));  // tables 1..D
     const size_t words = ((size_t)V + 3) / 4 * 16 * Wm;  // whole quads of vertices (k_bs_scan)
     const size_t o_fm0 = take(words);
@@ -939,7 +985,7 @@ struct Runner {
     shs.back().bytes = off;
     shs.back().D = D;
     shs.back().id = ++last_shared;
-    BsCtx h;
+    BsCtx& h = *h_bs;
     memset(&h, 0, sizeof(h));
     h.D = (uint32_t)D;
     for (int t = 1; t <= D; t++) h.tab[t] = (uint32_t*)(base + o_dist + (size_t)(t - 1) * V * Gp * 4);
@@ -981,7 +1027,7 @@ struct Runner {
     }
     for (int c = 0; c < BS_COLS; c++) h.cutc[c] = COST_INF;
     cudaStream_t st = eng->stream;
-    BsCtx* d_b = (BsCtx*)(base + o_b);
+    BsCtx* d_b = d_bs;
     int32_t* d_cols = (int32_t*)(base + o_cols);
     if (!eng->bs_ev[0]) {
       CK(cudaEventCreate(&eng->bs_ev[0]));
@@ -1007,10 +1053,20 @@ struct Runner {
     const int relax_blocks = eng->sms * std::max(1, std::min(occ, 4));
     const bool wide = V >= 600000;  // four vertices per scan thread
     const int scan_blocks = (int)std::min<int64_t>(eng->sms * 8, wide ? (V + 1023) / 1024 : (V + 255) / 256);
-    BsCtx hb;
+    // A hop-bounded search has D steps.  An unbounded one runs as a graph loop that its last
+    // relax step ends (looked at every six steps instead, it took 0.06 ms longer per lone
+    // query: two more round trips and the steps launched past the end); without graphs, or
+    // while launches are profiled, every six.
+    const bool looped = !D && eng->cfg.use_graphs && !eng->cfg.profile_kernels;
+    const BsCtx& hb = h;  // read back after the steps
     for (;;) {
-      // a hop-bounded search has D steps; an unbounded one is looked at every six
-      for (int i = 0; i < (D ? D : 6); i++) {
+      if (looped) {
+        cudaGraphExec_t ex;
+        s = search_graph(wide, scan_blocks, relax_blocks, &ex);
+        if (s != GST_OK) return s;
+        CK(cudaGraphLaunch(ex, st));
+      }
+      for (int i = 0; !looped && i < (D ? D : 6); i++) {
         if (D && i) {
           k_bs_copy<<<eng->sms * 4, 256, 0, st>>>(d_b, n4);
           launches++;
@@ -1020,20 +1076,23 @@ struct Runner {
                           : (pull ? k_bs_scan<1, true> : k_bs_scan<1, false>);
         scan<<<scan_blocks, 256, 0, st>>>(d_b, G);
         const int pe = prof_begin(PROF_BSRELAX);
-        if (pull) k_bs_relax<true><<<relax_blocks, 256, 0, st>>>(d_b, G);
-        else k_bs_relax<false><<<relax_blocks, 256, 0, st>>>(d_b, G);
+        if (pull) k_bs_relax<true><<<relax_blocks, 256, 0, st>>>(d_b, G, cudaGraphConditionalHandle{}, 0);
+        else k_bs_relax<false><<<relax_blocks, 256, 0, st>>>(d_b, G, cudaGraphConditionalHandle{}, 0);
         prof_end(pe);
         relax_launches++;
         launches += 2;
       }
       CK(cudaGetLastError());
-      CK(cudaMemcpyAsync(&hb, d_b, sizeof(BsCtx), cudaMemcpyDeviceToHost, st));
+      CK(cudaEventRecord(eng->bs_ev[1], st));
+      CK(cudaMemcpyAsync(h_bs, d_b, sizeof(BsCtx), cudaMemcpyDeviceToHost, st));
       cs.d2h += sizeof(BsCtx);
       CK(cudaStreamSynchronize(st));
       if (hb.done || D) break;
     }
-    CK(cudaEventRecord(eng->bs_ev[1], st));
-    CK(cudaEventSynchronize(eng->bs_ev[1]));
+    if (looped) {
+      relax_launches = (int64_t)hb.steps + 1;
+      launches += 2 * relax_launches;
+    }
     float ms = 0;
     cudaEventElapsedTime(&ms, eng->bs_ev[0], eng->bs_ev[1]);
     cs.bs_ms += ms;
@@ -1047,7 +1106,6 @@ struct Runner {
       shared_release(false);
       return GST_OK;
     }
-    S.d_b = d_b;
     S.Gp = Gp;
     S.dist = h.dist;
     for (int t = 0; t <= KMAX; t++) S.tab[t] = h.tab[t];
