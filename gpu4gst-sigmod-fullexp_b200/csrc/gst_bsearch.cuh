@@ -330,6 +330,7 @@ __global__ void __launch_bounds__(256, 4) k_bs_scan(BsCtx* b, DevGraph G) {
     }
     __syncthreads();
     uint32_t tw = s_base[0] + s_sum[0][wib] + sw - nw, tr = s_base[1] + s_sum[1][wib] + sr - nr;
+    // (by its size, V + E / chunk, the array holds every item of both lists)
     if (tw + nw + tr + nr > cap) atomicOr(&b->error, BS_ERR_ITEMS);
 #pragma unroll
     for (int i = 0; i < VPT; i++) {

@@ -2728,8 +2728,8 @@ gst_status noalloc_solve(int device, cudaStream_t st, int64_t V, int64_t E, cons
   const size_t o_fm1 = take(fm_bytes(V));
   const size_t o_snap = take(c.sssp_mask == 2u ? Vs * ds * 4 : 0);
   const size_t o_dh = take((size_t)nhb * Vs * ds * 4);
-  // four worklists (near and far, ping-pong) of at least 4V + 4096 items each
-  const size_t min_lists = 4 * (4 * Vs + 4096) * 16;
+  // four worklists (near and far, ping-pong) of at least 4V + 4064 items each
+  const size_t min_lists = 4 * (4 * Vs + 4064) * 16;
   if (off + min_lists > kNoallocScratchBytes) {
     char msg[200];
     snprintf(msg, sizeof msg,
