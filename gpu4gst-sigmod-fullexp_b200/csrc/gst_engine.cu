@@ -97,9 +97,8 @@ bool dense_rows(int64_t V, size_t rw, uint64_t rows, int boost) {
 // retry; at most 5/4 of the vertices, since every lost race for a row leaves one unused, or
 // one per vertex in the dense layout.  Most queries write rows for a few percent of the
 // vertices (their pruning keeps the DP near the optimal trees), but the heaviest k = 7 ones
-// overflow an eighth and then run twice, the second time with a search of their own (10 to
-// 22 of 155 ms of a batch of 32 over 4M vertices, the lost first run not counted: 129 ms
-// without).  No more than that: fresh memory costs its mapping and one clearing.
+// overflow an eighth and then run twice (with the second search 10 to 22 of 155 ms of a
+// batch of 32 over 4M vertices, the lost first run not counted: 129 ms without).  No more than that: fresh memory costs its mapping and one clearing.
 uint32_t pool_rows(int64_t V, size_t rw, size_t room, int boost) {
   const uint64_t more = std::max<uint64_t>((uint64_t)V / 8 * 3, kPoolBytes / (rw * 8));
   uint64_t r = std::max<uint64_t>(1u << 16, (uint64_t)V / 8);
@@ -387,6 +386,7 @@ struct Job {
   uint64_t ticket = 0;
   Clock::time_point t_submit;
   int boost = 0;                 // worklist capacity boost (capacity retries)
+  int pool_boost = 0;            // row pool boost (capacity retries)
   size_t rw = 0;
   int nhb = 0;                   // hop budgets of the one-label distances
   uint32_t ds = DIST_STRIDE;     // uint32 per distance row
@@ -574,7 +574,8 @@ struct Runner {
   // nothing where half the budget would not hold the query then
   uint32_t job_rows(const Job& j) const {
     const size_t room = std::min(kPoolRoom, budget / 64);
-    const uint32_t least = pool_rows(g->V, j.rw, 0, j.boost), r = pool_rows(g->V, j.rw, room, j.boost);
+    const uint32_t least = pool_rows(g->V, j.rw, 0, j.pool_boost),
+                   r = pool_rows(g->V, j.rw, room, j.pool_boost);
     if (r == least) return r;
     SlotMem tmp;
     const uint32_t cap = list_cap(g->V, g->E, j.rw, eng->cfg.split_degree, j.boost);
@@ -631,12 +632,13 @@ struct Runner {
     }
   }
   // Reserve a new arena of at least `need` bytes within the budget: at least 4 GB, and
-  // at least what is held already (geometric growth: mixed batches stop growing the
-  // arenas after their first few, since new physical memory costs ~8-9 ms per GB).
+  // at least what is held already, up to 16 GB (mixed batches stop growing the arenas after
+  // their first few, since new physical memory costs ~8-9 ms per GB).
   gst_status arena_grow(size_t need, bool* grown) {
     *grown = false;
     if (held + need > budget) return GST_OK;
-    const size_t chunk = std::max(need, std::min(std::max((size_t)4 << 30, held), budget - held));
+    const size_t chunk = std::max(
+        need, std::min(std::min(std::max((size_t)4 << 30, held), (size_t)16 << 30), budget - held));
     void* p = nullptr;
     const auto ta = Clock::now();
     CK(cudaMallocFromPoolAsync(&p, chunk, eng->pool, eng->stream));
@@ -814,7 +816,7 @@ struct Runner {
     // query wrote need clearing
     c.pool_cap = (uint32_t)std::min<uint64_t>(1u << 30, m.table_bytes / ((size_t)c.RW * 8));
     c.pool_n = 0;
-    if (dense_rows(g->V, (size_t)c.RW, c.pool_cap, j->boost)) {
+    if (dense_rows(g->V, (size_t)c.RW, c.pool_cap, j->pool_boost)) {
       c.rowmap = nullptr;
       c.pool_cap = (uint32_t)g->V;
     }
@@ -1319,8 +1321,11 @@ struct Runner {
         if (eng->cfg.verbose)
           fprintf(stderr, "[gst retry] k %d D %d: error bits 0x%x, pool %u of %u rows\n", c.k,
                   j->q.hop_bound, c.error, c.pool_n, c.pool_cap);
-        j->boost++;
-        j->ss = 0;  // a retry searches on its own
+        // each grows by itself: four times the worklists of a heavy query over 8.6M vertices
+        // are 4 GB that a retry for a full pool does not need
+        j->boost += list_full;
+        j->pool_boost += pool_full;
+        j->ss = 0;  // its table may be gone: a retry takes part in another search
         retry.push_back(j);
         continue;
       }
@@ -1907,12 +1912,12 @@ namespace {
 // would change it), refilling slots as queries finish; capacity overflows are re-run
 // with more room.  A job that does not fit the free memory yet does not hold back the
 // smaller ones behind it (a batch has no arrival order to keep).
-// A query the batch-shared search may serve: unbounded or of hop bound 1..KMAX, a first
-// attempt, not a cache fill, not every group in the group cache of its kind (those start
+// A query the batch-shared search may serve: unbounded or of hop bound 1..KMAX (a capacity
+// retry too: its own search took 50-100 ms over 8.6M vertices), not a cache fill, not every group in the group cache of its kind (those start
 // from exact distances; with only some cached, the shared table serves all of them).
 // Returns its kind (0 unbounded, else D), -1 if none.
 int shared_kind(const Runner& R, const Job* j) {
-  if (j->cache_dst || j->boost > 0 || j->ss) return -1;
+  if (j->cache_dst || j->ss) return -1;
   const int D = j->q.hop_bound;
   if (D == 0 || D > KMAX) return -1;
   const auto& hc = R.grp->hop_cache;
