@@ -27,9 +27,9 @@
 //                 T(u,X[,d+1]) with one atomicMin; an improved target marks its
 //                 row dirty (bitmap + compacted row list)
 //                 (code/TrimCDP-WB/include/mapper.cuh:366-413).
-//   control       one thread per query swaps worklists, advances the cost bucket
-//                 (near/far ordering), counts levels and detects the fixpoint
-//                 (replaces the grid barrier loop of mapper_enactor.cuh:158-246).
+//   control       in the last block of either kernel, one thread per query swaps
+//                 worklists, advances the cost bucket (near/far ordering), counts
+//                 levels and detects the fixpoint (replaces the grid barrier loop of mapper_enactor.cuh:158-246).
 // Pruning (every test compares with ub, the cost of a feasible tree, so no state of
 // an optimal tree is dropped):
 //   grow a state only if 2c <= ub (code/TrimCDP-WB/include/mapper_enactor.cuh /

@@ -8,7 +8,8 @@
 // Slot memory comes from the engine's stream-ordered memory pool and is admitted
 // against a memory budget by the size of each query's state table.
 //
-// The level loop is a fixed launch sequence (sssp, ctrl, rows, ctrl, grow, ctrl)
+// The level loop is a fixed launch sequence (rows, grow, each with its control step in its
+// last block; before them sssp, ctrl while some query searches its own distances)
 // that every resident query steps through together; each kernel reads its work
 // counts from the device-side contexts, so launches after a query finishes are
 // no-ops for it.  The host either issues a few levels ahead and then reads the
