@@ -34,6 +34,7 @@
 #include <cuda_runtime.h>
 
 #include "gst.h"
+#include "gst_admission.h"
 #include "gst_device.cuh"
 #include "gst_bsearch.cuh"
 
@@ -1470,7 +1471,7 @@ struct gst_server {
 };
 
 namespace {
-gst_status maybe_shared_search(Runner& R, std::deque<Job*>& pending);  // with the batch driver
+gst_status maybe_shared_search(Runner& R, std::deque<Job*>& pending, bool in_order);  // with the batch driver
 bool waits_for_search(const Runner& R, const Job* j);
 }  // namespace
 
@@ -1505,7 +1506,7 @@ void server_loop(gst_server* sv) {
           std::lock_guard<std::mutex> lk(sv->mu);
           snap = sv->pending;
         }
-        s_pre = maybe_shared_search(R, snap);
+        s_pre = maybe_shared_search(R, snap, true);
       }
       for (;;) {
         if (s_pre != GST_OK) break;
@@ -1949,26 +1950,21 @@ gst_status shared_search_kind(Runner& R, std::deque<Job*>& pending, int kind) {
   return R.shared_search(chunk, cols, kind);
 }
 
-// Before admitting: for every kind (unbounded, or one hop bound D) with an eligible query
-// waiting and fewer searched ones than there are free slots, search the groups of that
-// kind's first queries together (in order, up to BS_COLS distinct groups and BS_MAXQ
+// Before admitting: for every kind (unbounded, or one hop bound D) that is due (kinds_due;
+// in_order: the pass ends at the first query that waits for a search), search the groups of
+// that kind's first queries together (in order, up to BS_COLS distinct groups and BS_MAXQ
 // queries).  A lone query takes the same path: its search over k columns on these kernels
-// is faster than the per-query group-mask search on large graphs.  Kinds are searched in
-// the order their first queries wait.  An eligible query is admitted only once it has been
+// is faster than the per-query group-mask search on large graphs.  An eligible query is admitted only once it has been
 // part of a search: with one table per kind, and newcomers admitted on sight, 36 of a batch
 // of 100 queries searched alone, and most of 24 that arrived at a server while it took in
 // the first (90 ms for those over 1M vertices, 32 now; the 100 over 20k 9.5 and 8.8 ms).
-gst_status maybe_shared_search(Runner& R, std::deque<Job*>& pending) {
+gst_status maybe_shared_search(Runner& R, std::deque<Job*>& pending, bool in_order) {
   if (!R.eng->cfg.batch_search) return GST_OK;
   R.shared_release(false);
-  std::vector<int> kinds;
-  for (Job* j : pending) {
-    const int jk = shared_kind(R, j);
-    if (jk < 0 || std::find(kinds.begin(), kinds.end(), jk) != kinds.end()) continue;
-    int searched = 0;
-    for (const Runner::Shared& x : R.shs) searched += x.D == jk ? x.remaining : 0;
-    if (searched < R.max_slots - R.active) kinds.push_back(jk);
-  }
+  std::vector<Waiting> queue;
+  for (const Job* j : pending)
+    queue.push_back(j->ss == 1 ? Waiting{std::max(0, j->q.hop_bound), true} : Waiting{shared_kind(R, j), false});
+  const std::vector<int> kinds = kinds_due(queue, R.max_slots - R.active, in_order);
   for (int kind : kinds) {
     gst_status s = shared_search_kind(R, pending, kind);
     if (s != GST_OK) return s;
@@ -1987,7 +1983,7 @@ gst_status drive(Runner& R, std::deque<Job*>& pending, int B) {
   gst_status st = GST_OK;
   std::vector<Job*> done, retry;
   while (st == GST_OK && (!pending.empty() || R.active > 0)) {
-    st = maybe_shared_search(R, pending);
+    st = maybe_shared_search(R, pending, false);
     if (st != GST_OK) break;
     bool erased = false;
     for (auto it = pending.begin(); it != pending.end() && R.active < R.max_slots;) {
