@@ -65,6 +65,9 @@ namespace gst {
 
 constexpr int BS_COLS = 256;   // columns (distinct groups) of one shared search, at most
 constexpr int BS_MAXQ = MAXB;  // queries of one shared search, at most
+// The search finds distances up to here only: the relax kernel compares signed words, a cutoff
+// plus one among them.
+constexpr uint32_t BS_DIST_MAX = 0x7FFFFFFEu;
 
 struct BsCtx {
   uint32_t* dist;       // V x Gp distances, row v at dist + v * Gp
@@ -87,6 +90,7 @@ struct BsCtx {
   uint32_t in;          // fm[in] is scanned this step; fm[in ^ 1] takes its announcements
   uint32_t ann;         // the relax step announced something
   uint32_t done, steps, max_steps, error;
+  uint32_t far;         // some distance may be beyond BS_DIST_MAX (k_bs_far)
   uint32_t cut_pm;      // query cutoff: star x cut_pm / 1000
   uint32_t D;           // 0: unbounded distances; else the hop bound (rounds 0..D-1)
   uint32_t round;       // hop-bounded: the current round
@@ -445,7 +449,7 @@ __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G, cudaG
   if (b->done) return;
   const uint32_t Gp = b->Gp, Wm = b->Wm, nsec = Gp / 8u;
   for (uint32_t c = threadIdx.x; c < BS_COLS; c += blockDim.x)
-    s_c1[c >> 3][c & 7u] = c < Gp ? (int)(min(b->cutc[c], 0x7FFFFFFEu) + 1u) : 0;
+    s_c1[c >> 3][c & 7u] = c < Gp ? (int)(min(b->cutc[c], BS_DIST_MAX) + 1u) : 0;
   __syncthreads();
   // hop-bounded round r: sources in table r (the members at 0 for r = 0), targets in
   // table r + 1; a round announces only to a next one that pushes
@@ -657,6 +661,17 @@ __global__ void __launch_bounds__(256, 4) k_bs_relax(BsCtx* b, DevGraph G, cudaG
     bs_advance(b);
     if (in_loop) cudaGraphSetConditional(loop, b->done ? 0u : 1u);
   }
+}
+
+// Whether a distance of the table (n words) exceeds `most`, so that a path over one edge more
+// may have been too heavy for the search.
+__global__ void k_bs_far(BsCtx* b, int64_t n, uint32_t most) {
+  bool found = false;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t d = __ldcs(b->dist + i);
+    found = found || (d > most && d != COST_INF);
+  }
+  if (found) b->far = 1u;
 }
 
 // Hop-bounded tables (n4 = V x Gp / 4 uint4 per table).  Before round r >= 1:

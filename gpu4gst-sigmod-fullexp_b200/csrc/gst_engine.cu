@@ -1113,16 +1113,34 @@ struct Runner {
     S.Gp = Gp;
     S.dist = h.dist;
     for (int t = 0; t <= KMAX; t++) S.tab[t] = h.tab[t];
-    // a query's cutoff: the smallest final cutoff of its columns
+    // a query's cutoff: the smallest final cutoff of its columns, and no more than the largest
+    // distance the search tells apart (a star may cost more).  COST_INF, without a star, says
+    // that every distance is exact; should one have gone beyond that, the query searches on
+    // its own.  (Looked for only where paths can be that heavy.)
+    bool far = false;
+    std::vector<uint32_t> cuts;
+    for (Job* j : jobs) {
+      cuts.push_back(COST_INF);
+      for (int i = 0; i < j->q.k; i++) cuts.back() = std::min(cuts.back(), hb.cutc[hb.qcol[cuts.size() - 1][i]]);
+    }
+    if (std::count(cuts.begin(), cuts.end(), COST_INF) && (uint64_t)V * (uint64_t)g->max_w > BS_DIST_MAX && !D) {
+      k_bs_far<<<eng->sms * 8, 256, 0, st>>>(d_b, V * (int64_t)Gp, BS_DIST_MAX - (uint32_t)g->max_w);
+      CK(cudaGetLastError());
+      cs.launches++;
+      cs.bs_launches++;
+      CK(cudaMemcpyAsync(&h_bs->far, &d_b->far, 4, cudaMemcpyDeviceToHost, st));
+      CK(cudaStreamSynchronize(st));
+      cs.d2h += 4;
+      far = h_bs->far != 0;
+    }
     for (size_t q = 0; q < jobs.size(); q++) {
-      uint32_t cut = COST_INF;
-      for (int i = 0; i < jobs[q]->q.k; i++) cut = std::min(cut, hb.cutc[hb.qcol[q][i]]);
+      if (cuts[q] == COST_INF && far) continue;
       for (int i = 0; i < KMAX; i++) jobs[q]->ss_cols[i] = i < jobs[q]->q.k ? hb.qcol[q][i] : 0;
-      jobs[q]->ss_cut = cut;
+      jobs[q]->ss_cut = cuts[q] == COST_INF ? COST_INF : std::min(cuts[q], BS_DIST_MAX);
       jobs[q]->ss = 1;
       jobs[q]->ss_id = S.id;
+      S.remaining++;
     }
-    S.remaining = (int)jobs.size();
     return GST_OK;
   }
 
