@@ -1055,7 +1055,12 @@ struct Runner {
     int occ = 1;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bs_relax<false>, 256, 0);
     const int relax_blocks = eng->sms * std::max(1, std::min(occ, 4));
-    const bool wide = V >= 600000;  // four vertices per scan thread
+    // four vertices per scan thread from 2M vertices on, where a scan is bound by reading the
+    // announcement words: searches of 32 queries, k = 5, in ms with one and four: 5.0 / 5.8 at
+    // 141k vertices, 12.9 / 13.3 at 749k, 17.8 / 18.4 at 1.0M, 27.0 / 27.2 at 1.7M, 32.8 / 32.4
+    // at 2.4M, 78.7 / 76.1 at 4.6M; D = 4 lies the same way, a little further up (12.4 / 12.2 at
+    // 4.6M)
+    const bool wide = V >= 2000000;
     const int scan_blocks = (int)std::min<int64_t>(eng->sms * 8, wide ? (V + 1023) / 1024 : (V + 255) / 256);
     // A hop-bounded search has D steps.  An unbounded one runs as a graph loop that its last
     // relax step ends (looked at every six steps instead, it took 0.06 ms longer per lone

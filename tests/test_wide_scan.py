@@ -1,4 +1,4 @@
-"""The scan of four vertices a thread (graphs of 600,000 vertices on): vertex counts that leave 1, 2
+"""The scan of four vertices a thread (graphs of 2,000,000 vertices on): vertex counts that leave 1, 2
 and 3 vertices in the last quad, 1 to 8 mask words a vertex, pushing and pulling rounds of every
 hop bound, one and two edge classes, against queries that search on their own.  And the bounds
 D = 6 and 7 on small graphs, against the oracle."""
@@ -26,11 +26,11 @@ def _graph(V, m, seed):
 
 
 @pytest.mark.parametrize("V,m,columns,hops", [
-    (600_001, 1_200_000, 24, [None, 1, 2, 3, 4, 5, 6, 7, 8]),   # 1 mask word
-    (600_002, 1_200_000, 84, [None, 3, 4]),                     # 3
-    (600_003, 1_200_000, 136, [None, 2, 5]),                    # 5
-    (600_003, 1_200_000, 240, [None, 4, 8]),                    # 8
-    (600_001, 8_500_000, 240, [None]),                          # 8, two edge classes
+    (2_000_001, 1_200_000, 24, [None, 1, 2, 3, 4, 5, 6, 7, 8]),   # 1 mask word
+    (2_000_002, 1_200_000, 84, [None, 3, 4]),                     # 3
+    (2_000_003, 1_200_000, 136, [None, 2, 5]),                    # 5
+    (2_000_003, 1_200_000, 240, [None, 4, 8]),                    # 8
+    (2_000_001, 8_500_000, 240, [None]),                          # 8, two edge classes
 ])
 def test_queries_keep_their_cost(V, m, columns, hops):
     g = _graph(V, m, V + columns)
