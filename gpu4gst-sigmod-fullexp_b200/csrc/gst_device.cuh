@@ -101,11 +101,13 @@ enum ErrBits : uint32_t { ERR_QCAP = 1, ERR_FARCAP = 2, ERR_ROWCAP = 4, ERR_TIME
 constexpr uint32_t ROW_NONE = 0xFFFFFFFFu;
 
 // Light-edge index: per vertex, the number of edges of weight <= widx_threshold(t) << wsh
-// for t < WIDX, thresholds 1, 2, 3, 4, 6, 8, 12, ..., 192, 256 (each step x1.5 or
-// x1.33), so that one load bounds the edges a relaxation under a weight limit
-// needs, over-counting by at most a third.  The graph's shift wsh puts the thresholds
-// where its weights are: the smallest with 256 << wsh >= twice the median weight (0 up
-// to a median of 128; a few heavy outliers do not move it).  With weights of 1..10^6
+// for t < WIDX, thresholds 1, 2, 3, 4, 6, 8, 12, ..., 192, 256, so that one load bounds the
+// edges a relaxation under a weight limit needs.  It returns those up to the next threshold
+// (less than 1.5 times a limit above 2 << wsh, at most twice one above 1 << wsh, 1 << wsh for
+// the smaller ones; all edges for limits above the last threshold); the per-edge tests drop
+// the rest.  The graph's shift wsh puts the thresholds where its weights are: the smallest with
+// 256 << wsh >= twice the median weight (0 up to a median of 128; a few heavy outliers do not
+// move it).  With weights of 1..10^6
 // (wsh = 12), where unscaled thresholds made every relaxation read the whole list,
 // 12 queries over 141k vertices relax 125 M edges without the shift and 25 M with it
 // (grow 4.6 to 3.1 ms, the call 15.2 to 13.6 ms).

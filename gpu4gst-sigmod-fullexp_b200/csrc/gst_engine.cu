@@ -89,18 +89,19 @@ size_t fm_bytes(int64_t V) { return ((size_t)V + 15) / 16 * 16; }
 
 // Whether a table of at least V rows is laid out densely (one row per vertex, no map):
 // where it is small or has few vertices (clearing it costs less than the map's extra
-// reads), and after a capacity retry.
+// reads), and after a retry for a full pool.
 bool dense_rows(int64_t V, size_t rw, uint64_t rows, int boost) {
   return rows >= (uint64_t)V &&
          ((size_t)V * rw * 8 <= kDenseBytes || V <= kDenseVertices || boost > 0);
 }
 // Rows of a query's row pool: an eighth of the vertices (at least 64k rows); where `room`
-// bytes hold more, three eighths of them or 256 MB of rows; four times more per capacity
-// retry; at most 5/4 of the vertices, since every lost race for a row leaves one unused, or
+// bytes hold more, three eighths of them or 256 MB of rows; four times more per retry for a
+// full pool; at most 5/4 of the vertices, since every lost race for a row leaves one unused, or
 // one per vertex in the dense layout.  Most queries write rows for a few percent of the
 // vertices (their pruning keeps the DP near the optimal trees), but the heaviest k = 7 ones
-// overflow an eighth and then run twice (with the second search 10 to 22 of 155 ms of a
-// batch of 32 over 4M vertices, the lost first run not counted: 129 ms without).  No more than that: fresh memory costs its mapping and one clearing.
+// overflow an eighth and then run twice: a batch of 32 over 4M vertices with one of them took
+// 155 ms with pools of an eighth and 129 ms with these.  Larger pools map more memory and
+// clear it once: with up to 2 GB of rows instead of 1.5 the first call took 0.8 s longer.
 uint32_t pool_rows(int64_t V, size_t rw, size_t room, int boost) {
   const uint64_t more = std::max<uint64_t>((uint64_t)V / 8 * 3, kPoolBytes / (rw * 8));
   uint64_t r = std::max<uint64_t>(1u << 16, (uint64_t)V / 8);
@@ -156,9 +157,10 @@ int hop_budgets(int D) { return D > 1 ? std::min(D - 1, HOP_BUDGETS_MAX) : 0; }
 
 // Worklist capacity.  A level appends at most one item per edge chunk of every
 // state it settles, which in the worst case is every cell of the slab; queries
-// use a small fraction of that, so a slot starts at 8 items per vertex, from 1M vertices on
-// 4 (the heaviest k = 7 queries over 4M vertices fill 1.04), and a query that overflows is
-// re-run with four times the room (up to the worst case).
+// use a small fraction of that, so a slot starts at 8 items per vertex up to 1M vertices, stays
+// at 8M items up to 2M and has 4 per vertex beyond (the heaviest k = 7 queries over 4M vertices
+// fill 1.04), and a query that overflows is re-run with four times the room (up to the worst
+// case).
 uint32_t list_cap(int64_t V, int64_t E, size_t rw, int split, int boost) {
   const uint64_t worst = std::min<uint64_t>((uint64_t)V * rw + (uint64_t)E / split * rw + 4096,
                                             (1ull << 31));
@@ -946,12 +948,6 @@ struct Runner {
   // cutoff; without memory for the tables, or when the search reports an error, the jobs
   // search on their own (ss = 2).
   gst_status shared_search(const std::vector<Job*>& jobs, const std::vector<int32_t>& cols, int D) {
-    gst_status s = GST_OK;
-    if (n_aq) {  // nothing admitted reads memory that is taken below
-      s = start_admitted();
-      if (s != GST_OK) return s;
-      CK(cudaStreamSynchronize(eng->stream));  // h_aq is free again
-    }
     for (Job* j : jobs) j->ss = 2;  // until the search has succeeded
     const int64_t V = g->V;
     const uint32_t ncols = (uint32_t)cols.size();
@@ -979,7 +975,7 @@ struct Runner {
     const size_t o_items = take((size_t)item_cap * 8);
     const size_t o_cols = take((size_t)BS_COLS * 4);
     void* p = nullptr;
-    s = slot_memory(off, &p);
+    gst_status s = slot_memory(off, &p);
     if (s != GST_OK) return s;
     if (!p) return GST_OK;  // no room: the queries search on their own
     unsigned char* base = (unsigned char*)p;
@@ -1938,9 +1934,10 @@ namespace {
 // with more room.  A job that does not fit the free memory yet does not hold back the
 // smaller ones behind it (a batch has no arrival order to keep).
 // A query the batch-shared search may serve: unbounded or of hop bound 1..KMAX (a capacity
-// retry too: its own search took 50-100 ms over 8.6M vertices), not a cache fill, not every group in the group cache of its kind (those start
-// from exact distances; with only some cached, the shared table serves all of them).
-// Returns its kind (0 unbounded, else D), -1 if none.
+// retry too: its own search took 50-100 ms over 8.6M vertices), not a cache fill, not every
+// group in the group cache of its kind (those start from exact distances; with only some
+// cached, the shared table serves all of them).  Returns its kind (0 unbounded, else D), -1
+// if none or once one has covered it.
 int shared_kind(const Runner& R, const Job* j) {
   if (j->cache_dst || j->ss) return -1;
   const int D = j->q.hop_bound;
@@ -1983,6 +1980,11 @@ gst_status shared_search_kind(Runner& R, std::deque<Job*>& pending, int kind) {
 // the first (90 ms for those over 1M vertices, 32 now; the 100 over 20k 9.5 and 8.8 ms).
 gst_status maybe_shared_search(Runner& R, std::deque<Job*>& pending, bool in_order) {
   if (!R.eng->cfg.batch_search) return GST_OK;
+  // every query admitted before has started (run() follows each admission pass that took
+  // one), so none still has to read from a table that is given back or memory taken here
+#ifdef GST_CHECKED
+  if (R.n_aq) return fail(R.eng, GST_DEVICE_ERROR, "search: admitted queries have not started");
+#endif
   R.shared_release(false);
   std::vector<Waiting> queue;
   for (const Job* j : pending)

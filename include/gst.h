@@ -172,16 +172,18 @@ gst_status gst_groups_destroy(gst_groups* grp);
  * up to max_bytes (4 x V bytes per group; when the list holds more groups than fit,
  * the first ones are kept; groups of earlier calls that this call does not list are
  * replaced least recently used first).  Unbounded queries whose groups are all cached
- * then skip the distance search; with some of their groups cached, the search runs for
- * the others only.  A different max_bytes drops the cache first;
+ * then skip the distance search.  With only some of their groups cached they take part in
+ * a shared search like uncached ones (cfg.batch_search = 0: their own search runs for the
+ * other groups only).  A different max_bytes drops the cache first;
  * max_bytes = 0 frees it.  *n_cached (optional) = listed groups now cached. */
 gst_status gst_groups_cache_warm(gst_groups* grp, int32_t n, const int32_t* group_ids,
                                  int64_t max_bytes, int32_t* n_cached);
 /* The same for queries with hop bound hop_bound (1..30): per group, the cheapest paths
  * of at most h edges to every vertex for every hop budget the engine bounds with
  * (4 x V x (min(hop_bound-1, 7) + 1) bytes per group).  A hop-bounded query with that
- * bound whose groups are all cached skips the distance search; with some cached, the
- * search runs for the others only.  One hop bound at a time: warming with another (or
+ * bound whose groups are all cached skips the distance search; with only some cached it
+ * takes part in a shared search (D <= 8; else its own search runs for the other groups
+ * only).  One hop bound at a time: warming with another (or
  * another max_bytes) drops the hop cache first. */
 gst_status gst_groups_cache_warm_hop(gst_groups* grp, int32_t n, const int32_t* group_ids,
                                      int32_t hop_bound, int64_t max_bytes, int32_t* n_cached);
