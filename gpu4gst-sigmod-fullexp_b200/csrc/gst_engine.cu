@@ -636,8 +636,9 @@ struct Runner {
     }
   }
   // Reserve a new arena of at least `need` bytes within the budget: at least 4 GB, and
-  // at least what is held already, up to 16 GB (mixed batches stop growing the arenas after
-  // their first few, since new physical memory costs ~8-9 ms per GB).
+  // at least what is held already, up to 16 GB.  (Mapping it takes 6 ms per GB where the device
+  // has cleared pages and up to 100 where it has not; mixed batches over 4M vertices map 70 GB
+  // in their first call and 17 GB in their third and sixth.)
   gst_status arena_grow(size_t need, bool* grown) {
     *grown = false;
     if (held + need > budget) return GST_OK;
